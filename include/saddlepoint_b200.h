@@ -232,7 +232,9 @@ int sp_solver_kernel_timing(sp_solver *s, int id, int64_t *launches, double *tot
 double sp_solver_bytes_per_iteration(sp_solver *s);
 /* Which engine runs each fused pass of the solver (chosen at creation from the
  * problem's size, or SP_PASS_ENGINE): out[0] primal FP64, out[1] primal FP32,
- * out[2] dual FP64, out[3] dual FP32 (the FP32 entries apply to the mixed form). */
+ * out[2] dual FP64, out[3] dual FP32 (the FP32 entries apply to the mixed form). A small
+ * LP's iterations run on chip, several epochs to a launch; the engines named here then run
+ * its passes only where sp_solver_set_timing has them launched one by one. */
 enum { SP_ENGINE_TILES = 0, SP_ENGINE_STREAM = 1, SP_ENGINE_SELL = 2 };
 int sp_solver_engines(sp_solver *s, int32_t out[4]);
 /* The floor a pass's random gathers set: the average time of a kernel that does only
@@ -241,7 +243,8 @@ int sp_solver_engines(sp_solver *s, int32_t out[4]);
  * over `reps` launches after one warm-up. For reading a pass's time against. */
 int sp_solver_gather_floor(sp_solver *s, int pass, int fp32, int reps, double *ms_per_launch);
 /* Kernel launches of one epoch of check_every iterations, counted from the
- * kernel nodes of its CUDA graph (the graph is built if it does not exist yet). */
+ * kernel nodes of its CUDA graph (the graph is built if it does not exist yet); for a small
+ * LP on chip, the launches that its epochs share (one, in the mixed form two). */
 int sp_solver_epoch_kernels(sp_solver *s, int64_t *count);
 /* Downloads the scaled problem the solver built on the device (ScaledProblem,
  * scaling.rs:36-50): A' and A'ᵀ in CSR, c', lc', uc', lv', uv', the row and

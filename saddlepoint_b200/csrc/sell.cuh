@@ -386,25 +386,6 @@ namespace sp {
 // so adding a contribution that started from +0.0 gives the bits the tile engine's
 // in-place accumulation gives.
 
-template <int G, unsigned F32>
-struct SlotSums {
-    float f[G];
-    double d[G];
-    __device__ __forceinline__ void clear() {
-#pragma unroll
-        for (int q = 0; q < G; ++q) { f[q] = -0.0f; d[q] = -0.0; }
-    }
-    template <class ST>
-    __device__ __forceinline__ void add(const ST (&p)[G]) {
-#pragma unroll
-        for (int q = 0; q < G; ++q) {
-            if ((F32 >> q) & 1u) f[q] += float(p[q]);
-            else d[q] += double(p[q]);
-        }
-    }
-    __device__ __forceinline__ double get(int q) const { return ((F32 >> q) & 1u) ? double(f[q]) : d[q]; }
-};
-
 // One row's epilogue with its partials from zero, stored as its contributions.
 template <class Op>
 __device__ __forceinline__ void row_contrib(const Op &op, int r, const double (&sum)[Op::G],

@@ -1005,6 +1005,165 @@ int choose_engines(sp_solver *s) {
     return SP_OK;
 }
 
+// ------------------------------------------------------------------ the on-chip engine
+
+constexpr int RES_SMEM_MAX = (int)STREAM_SMEM_MAX - 4096;  // dynamic shared memory of a CTA, beside ResShared
+static_assert(sizeof(ResShared) <= 4096, "the static part fits beside it");
+constexpr uint64_t RES_MAX_EPOCHS = 16;  // epochs of one launch at most
+
+template <int NC>
+ResKernel res_kernel_of(bool lo, bool entries) {
+    return lo ? (entries ? k_res_epochs<NC, true, true> : k_res_epochs<NC, true, false>)
+              : (entries ? k_res_epochs<NC, false, true> : k_res_epochs<NC, false, false>);
+}
+
+// Launches one of the engine's kernels as one cluster.
+int res_launch(const sp_solver *s, const ResLaunch &l, unsigned long long n) {
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3((unsigned)s->res_ctas);
+    cfg.blockDim = dim3(RES_BT);
+    cfg.dynamicSmemBytes = (size_t)l.smem;
+    cfg.stream = s->ctx->stream;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = (unsigned)s->res_ctas;
+    at[0].val.clusterDim.y = 1;
+    at[0].val.clusterDim.z = 1;
+    if (s->res_ctas > 1) {
+        cfg.attrs = at;
+        cfg.numAttrs = 1;
+    }
+    SP_CUDA_TRY(cudaLaunchKernelEx(&cfg, l.f, s->res, n));
+    return SP_OK;
+}
+
+// Enqueues epochs until the state's total is `until`: in the mixed form the FP32 phase's
+// kernel and then the FP64 one's.
+int res_launch_epochs(const sp_solver *s, uint64_t until) {
+    int rc = SP_OK;
+    if (s->mixed) rc = res_launch(s, s->res_epochs[1], until);
+    return rc ? rc : res_launch(s, s->res_epochs[0], until);
+}
+
+// CTAs of the cluster for an LP of this size: one where it fits and has under 3200 nonzeros.
+// There the cluster's barrier (about 450 clocks, against 40) costs what its seven more SMs
+// give (µs per iteration, checks included, one CTA / eight: 1,809 nonzeros 1.55 / 1.95, 3,248
+// nonzeros 2.07 / 2.07).
+int res_cluster_of(int64_t m, int64_t n, int64_t nnz) {
+    return nnz < 3200 && n <= RES_PT && m <= RES_PA ? 1 : RES_CLUSTER;
+}
+
+// Sets the on-chip engine up for the scaled problem where the LP fits it: no row longer than a
+// tile, and its vectors in the CTAs' shared memory. rp_t: the row pointers of A'ᵀ.
+int res_build(sp_solver *s, const sp_lp *lp, const std::vector<int> &rp_t) {
+    const int64_t m = s->m, n = s->n, nnz = s->nnz;
+    const char *eng = getenv("SP_PASS_ENGINE");
+    if (eng && strcmp(eng, "resident")) return SP_OK;  // another engine is asked for
+    if (nnz >= SMALL_NNZ || nnz == 0 || m > RES_MAX_ROWS || n > RES_MAX_ROWS || m < 1 || n < 1) return SP_OK;
+    const int ctas = res_cluster_of(m, n, nnz);
+    if (s->A.nlong || s->AT.nlong || m > (int64_t)RES_PA * ctas || n > (int64_t)RES_PT * ctas) return SP_OK;
+    ResPlan PA, PT;
+    res_plan(lp->a.row_ptr, (int)m, ctas, &PA);
+    res_plan(rp_t.data(), (int)n, ctas, &PT);
+    if (PA.most_rows > RES_PA || PT.most_rows > RES_PT) return SP_OK;
+    ResArgs &a = s->res;
+    auto sizes = [](ResSrc &q, const ResPlan &P, const DevCsr &M) {
+        q.rows = (int)M.nrows;
+        q.heavy = P.heavy;
+        q.ntiles = M.ntiles;
+        q.most_rows = P.most_rows;
+        q.most_slots = P.most_slots;
+        q.most_tasks = P.most_tasks;
+        q.rp = M.rp;
+        q.tiles = M.tiles;
+    };
+    sizes(a.A, PA, s->A);
+    sizes(a.T, PT, s->AT);
+    // the kernels: entries in shared memory where they fit (FP64, and the FP32 phase)
+    const bool one = ctas == 1;
+    for (int lo = 0; lo < (s->mixed ? 2 : 1); ++lo) {
+        const int in = res_solver_places(a.A, a.T, lo, true).total, out = res_solver_places(a.A, a.T, lo, false).total;
+        if (out > RES_SMEM_MAX) return SP_OK;
+        const bool fits = in <= RES_SMEM_MAX;
+        s->res_epochs[lo] = ResLaunch{one ? res_kernel_of<1>(lo, fits) : res_kernel_of<RES_CLUSTER>(lo, fits), fits ? in : out};
+        if (lo == 0)
+            s->res_power = ResLaunch{one ? (fits ? k_res_power<1, true> : k_res_power<1, false>)
+                                         : (fits ? k_res_power<RES_CLUSTER, true> : k_res_power<RES_CLUSTER, false>),
+                                     fits ? in : out};
+    }
+    for (const ResLaunch *l : {&s->res_epochs[0], &s->res_epochs[1], &s->res_power})
+        if (l->f) SP_CUDA_TRY(cudaFuncSetAttribute((const void *)l->f, cudaFuncAttributeMaxDynamicSharedMemorySize, RES_SMEM_MAX));
+    // one upload for the plans, one allocation for them, the slots and the scratch
+    std::vector<unsigned char> h;
+    size_t bytes = 0;
+    auto room = [&](size_t b) {
+        const size_t at = bytes;
+        bytes += (b + 255) & ~size_t(255);
+        return at;
+    };
+    auto vec = [&](const auto &v) {
+        const size_t b = v.size() * sizeof(v[0]), at = room(b);
+        h.resize(bytes);
+        if (b) memcpy(h.data() + at, v.data(), b);
+        return at;
+    };
+    struct Off {
+        size_t perm, inv, tasks, wt, p0, s0, ci, v, v32;
+    } oa{}, ot{};
+    auto plan = [&](const ResPlan &P, Off *o) {
+        o->perm = vec(P.perm);
+        o->inv = vec(P.inv);
+        o->tasks = vec(P.tasks);
+        o->wt = vec(P.wt);
+        o->p0 = vec(P.p0);
+        o->s0 = vec(P.s0);
+    };
+    plan(PA, &oa);
+    plan(PT, &ot);
+    const size_t up = bytes;
+    auto slots = [&](const ResPlan &P, Off *o) {
+        o->ci = room(sizeof(uint16_t) * (size_t)P.slots);
+        o->v = room(sizeof(double) * (size_t)P.slots);
+        o->v32 = s->mixed ? room(sizeof(float) * (size_t)P.slots) : 0;
+    };
+    slots(PA, &oa);
+    slots(PT, &ot);
+    const size_t vecs = room(sizeof(double) * (3 * (size_t)n + 2 * (size_t)m));
+    const size_t contrib = room(sizeof(double) * (13 * (size_t)n + 8 * (size_t)m));
+    cudaStream_t st = s->ctx->stream;
+    int rc;
+    if ((rc = dmalloc(&s->res_mem, bytes))) return rc;
+    unsigned char *d = (unsigned char *)s->res_mem;
+    SP_CUDA_TRY(cudaMemcpyAsync(d, h.data(), up, cudaMemcpyHostToDevice, st));
+    auto place = [&](ResSrc &q, const Off &o) {
+        q.tasks = (const ResTask *)(d + o.tasks);
+        q.wt = (const int *)(d + o.wt);
+        q.p0 = (const int *)(d + o.p0);
+        q.s0 = (const int *)(d + o.s0);
+        q.perm = (const uint16_t *)(d + o.perm);
+        q.ci = (uint16_t *)(d + o.ci);
+        q.v = (double *)(d + o.v);
+        q.v32 = s->mixed ? (float *)(d + o.v32) : nullptr;
+    };
+    place(a.A, oa);
+    place(a.T, ot);
+    double *v = (double *)(d + vecs);
+    a.vec = ResVecs{v, v + n, v + 2 * n, v + 3 * n, v + 3 * n + m};
+    a.contrib = (double *)(d + contrib);
+    a.ppart = s->ppart;
+    a.trace = s->d_trace;
+    a.trace_cap = (long long)s->trace_cap;
+    a.mixed = s->mixed;
+    a.g = ptrs_of(s);
+    const int ta = (int)PA.tasks.size(), tt = (int)PT.tasks.size(), W = NT / 32;
+    k_res_fill<<<(ta + W - 1) / W, NT, 0, st>>>(a.A, ctas, ta, (int)n, (const uint16_t *)(d + ot.inv), s->A.ci, s->A.v);
+    k_res_fill<<<(tt + W - 1) / W, NT, 0, st>>>(a.T, ctas, tt, (int)m, (const uint16_t *)(d + oa.inv), s->AT.ci, s->AT.v);
+    SP_CUDA_TRY(cudaGetLastError());
+    SP_CUDA_TRY(cudaStreamSynchronize(st));  // the host's copy of the plans ends here
+    s->res_ctas = ctas;
+    return SP_OK;
+}
+
 // Launches the primal pass of iteration i with the given role. MID iterations go
 // through the stream engine when it is on (in the mixed form one launch per
 // precision; the one that does not match the device state returns at once).
@@ -1212,6 +1371,7 @@ void solver_release(sp_solver *s) {
         cudaEventDestroy(s->join);
     }
     cudaStream_t fst = s->ctx->stream;
+    dfree(s->res_mem, fst);
     free_csr(&s->A, fst);
     free_csr(&s->AT, fst);
     free_sell(&s->sellA, fst);
@@ -1644,17 +1804,23 @@ int power_iteration(sp_solver *s) {  // Solver::estimate_norm (solver.rs:215-242
         s->norm_est = 1.0;
         return SP_OK;
     }
-    k_power_fill<<<grid_of(s->ctx, s->n), NT, 0, st>>>(s->pv, s->n);
-    k_power_init<<<1, NT, 0, st>>>(s->n, s->ppart);
-    k_power_start<<<1, 32, 0, st>>>(s->ppart, s->d_st);
+    if (!s->res_ctas) {
+        k_power_fill<<<grid_of(s->ctx, s->n), NT, 0, st>>>(s->pv, s->n);
+        k_power_init<<<1, NT, 0, st>>>(s->n, s->ppart);
+        k_power_start<<<1, 32, 0, st>>>(s->ppart, s->d_st);
+    }
     const uint64_t maxit = s->prm.power_iterations;
     PowerA a{s->A.rp, s->A.ci, s->A.v, s->A.tiles, s->pv, s->ptmp, s->d_st, 0.0};
     PowerT t{s->AT.rp, s->AT.ci, s->AT.v, s->AT.tiles, s->ptmp, s->pv, s->ppart, s->d_st};
     const uint64_t chunk = 8;
+    if (s->res_ctas && maxit > 0) {  // a small LP: all iterations in one launch
+        const int rc = res_launch(s, s->res_power, maxit);
+        if (rc) return rc;
+    }
     DevState h{};  // with no iterations, λ stays 0 as in the reference
     for (uint64_t done_it = 0; done_it < maxit;) {
-        const uint64_t c = std::min(chunk, maxit - done_it);
-        for (uint64_t q = 0; q < c; ++q) {
+        const uint64_t c = s->res_ctas ? maxit : std::min(chunk, maxit - done_it);
+        for (uint64_t q = 0; q < c && !s->res_ctas; ++q) {
             // A'·v on the SELL copy where the dual passes have one (the same bits; 0.21 ms on
             // the tile engine for the 40M LP), else on the tile engine
             if (s->sellA.ok) launch_sell(s, s->sellA, st, a);
@@ -1811,7 +1977,6 @@ extern "C" int sp_solver_create(sp_ctx *ctx, const sp_lp *lp, const sp_solver_pa
     if ((rc = scale_on_device(s, lp, rp_t, &side))) return cleanup(rc);
     // the host's tile plan of A'ᵀ while the GPU runs the scaling sweeps
     if ((rc = plan_transpose(s, rp_t))) return cleanup(rc);
-    rp_t = std::vector<int>();
     stage("scaling");
     if (s->mixed) {
         if ((rc = dalloc(&s->A.v32, s->nnz)) || (rc = dalloc(&s->AT.v32, s->nnz))) return cleanup(rc);
@@ -1835,6 +2000,8 @@ extern "C" int sp_solver_create(sp_ctx *ctx, const sp_lp *lp, const sp_solver_pa
     SP_CUDA_TRY(cudaMallocHost(&s->h_st, sizeof(DevState) * (SolverLookahead + 2)));
     if ((rc = set_smem_limits())) return cleanup(rc);
     if ((rc = choose_engines(s))) return cleanup(rc);
+    if ((rc = res_build(s, lp, rp_t))) return cleanup(rc);
+    rp_t = std::vector<int>();
     stage("engines");
     // ‖A'‖₂ and η (solver.rs:316), while the second stream forms the norms
     if ((rc = power_iteration(s))) return cleanup(rc);
@@ -1899,9 +2066,32 @@ int epoch_graph(sp_solver *s, int E, cudaGraphExec_t *g) {
     return SP_OK;
 }
 
+// Iterations of the next epoch (0: the iteration limit is reached).
+uint64_t next_epoch(const sp_solver *s) {
+    return std::min<uint64_t>(s->prm.check_every, s->prm.max_iterations - std::min(s->launched, s->prm.max_iterations));
+}
+
+// Whether epochs run on the on-chip engine, which takes several in one launch.
+bool res_epochs_on(const sp_solver *s) { return s->res_ctas > 0 && s->timing_every == 0; }
+
+// Enqueues the next `n` epochs (fewer at the iteration limit) on the on-chip engine.
+int res_launch_next(sp_solver *s, uint64_t n) {
+    uint64_t its = 0, k = 0;
+    for (; k < n; ++k) {
+        const uint64_t E = next_epoch(s);
+        if (E == 0) break;
+        s->launched += E;
+        its += E;
+    }
+    const int rc = k ? res_launch_epochs(s, s->launched) : SP_OK;
+    if (rc) s->launched -= its;
+    return rc;
+}
+
 // Enqueues one epoch (graph, or direct launches when timing samples are due).
 int launch_epoch(sp_solver *s, int E) {
     cudaStream_t st = s->ctx->stream;
+    if (res_epochs_on(s)) return res_launch_next(s, 1);
     if (s->timing_every > 0) {
         enqueue_epoch(s, E, st, true);
     } else {
@@ -1939,8 +2129,14 @@ extern "C" int sp_solver_run_epochs(sp_solver *s, uint64_t epochs) {
     int rc = enter(s->ctx);
     if (rc) return rc;
     for (uint64_t e = 0; e < epochs; ++e) {
-        const uint64_t E = std::min<uint64_t>(s->prm.check_every, s->prm.max_iterations - std::min(s->launched, s->prm.max_iterations));
+        const uint64_t E = next_epoch(s);
         if (E == 0) break;
+        if (res_epochs_on(s)) {
+            const uint64_t n = std::min(epochs - e, RES_MAX_EPOCHS);
+            if ((rc = res_launch_next(s, n))) return rc;
+            e += n - 1;
+            continue;
+        }
         if ((rc = launch_epoch(s, (int)E))) return rc;
     }
     return SP_OK;
@@ -1976,19 +2172,27 @@ extern "C" int sp_solver_solve(sp_solver *s, sp_solution_info *info) {
         events.e.push_back(e);
     }
     std::vector<cudaEvent_t> &ev = events.e;
+    // the on-chip engine takes a growing number of epochs per launch where nothing is
+    // observed between them (a time limit and the progress log are, once per epoch)
+    const bool several = res_epochs_on(s) && limit <= 0 && s->prm.log_every_checks == 0;
+    uint64_t burst = 1;
     uint64_t queued = 0, seen = 0;
     bool stop = false;
     DevState last{};
     uint64_t logged_checks = 0;
     while (!stop) {
         while (!stop && queued - seen < (uint64_t)SolverLookahead + 1) {
-            const uint64_t E = std::min<uint64_t>(s->prm.check_every,
-                                                  s->prm.max_iterations - std::min(s->launched, s->prm.max_iterations));
+            const uint64_t E = next_epoch(s);
             if (E == 0) {
                 stop = queued == seen;
                 break;
             }
-            if ((rc = launch_epoch(s, (int)E))) return rc;
+            if (several) {
+                if ((rc = res_launch_next(s, burst))) return rc;
+                burst = std::min(2 * burst, RES_MAX_EPOCHS);
+            } else if ((rc = launch_epoch(s, (int)E))) {
+                return rc;
+            }
             const int slot = (int)(queued % ev.size());
             SP_CUDA_TRY(cudaMemcpyAsync(&s->h_st[slot], s->d_st, sizeof(DevState), cudaMemcpyDeviceToHost, st));
             SP_CUDA_TRY(cudaEventRecord(ev[slot], st));
@@ -2174,6 +2378,10 @@ extern "C" int sp_solver_epoch_kernels(sp_solver *s, int64_t *count) {
     if (!s || !count) return SP_ERR_INVALID;
     int rc = enter(s->ctx);
     if (rc) return rc;
+    if (s->res_ctas) {  // one launch (of up to RES_MAX_EPOCHS epochs) per precision
+        *count = s->mixed ? 2 : 1;
+        return SP_OK;
+    }
     const int E = (int)std::max<uint64_t>(1, s->prm.check_every);
     cudaGraphExec_t g;
     if ((rc = epoch_graph(s, E, &g))) return rc;

@@ -253,7 +253,7 @@ struct DualPass {
     }
     __device__ __forceinline__ void row(int r, const double (&sum)[G], double *part, const Pre &in) const {
         const double a = sum[0], yi = in.y;
-        const double v = a - yi / sc.sigma;                              // cpu lib.rs:171
+        const double v = a - div_by_positive(yi, sc.sigma);              // cpu lib.rs:171
         const double yt = yi - sc.sigma * (a - clampd(v, in.lc, in.uc)); // cpu lib.rs:172
         if constexpr (MODE == 0) {
             const double yn = halpern(yi, yt, in.ya, sc.w, sc.rho);

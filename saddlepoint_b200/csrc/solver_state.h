@@ -5,11 +5,17 @@
 #include <vector>
 
 #include "internal.cuh"
+#include "resident.cuh"
 #include "sell.cuh"
 #include "stream.cuh"
 
 namespace sp {
 constexpr int SolverLookahead = 2;  // epochs queued ahead of the state the host has read
+using ResKernel = void (*)(ResArgs, unsigned long long);
+struct ResLaunch {  // a kernel of the on-chip engine and its dynamic shared memory
+    ResKernel f = nullptr;
+    int smem = 0;
+};
 struct TimingSample {
     cudaEvent_t e0, e1, e2;  // before P, between P and D, after D
 };
@@ -26,6 +32,12 @@ struct sp_solver {
     sp::SellMat sellA, sellAT;  // SELL copies of A' (dual pass) and A'ᵀ (primal pass), when used
     cudaStream_t aux = nullptr;  // second stream of a SELL pass: its warp rows beside its windows
     cudaEvent_t fork = nullptr, join = nullptr;
+    // a small LP's on-chip engine (resident.cuh): CTAs of its cluster (0: not used), its kernels'
+    // arguments, and the memory of its plan and slots
+    int res_ctas = 0;
+    sp::ResArgs res{};
+    sp::ResLaunch res_epochs[2], res_power;  // epochs in FP64 and of the FP32 phase
+    void *res_mem = nullptr;
     double *contrib = nullptr;   // [NP_D][m] row contributions of the check's dual pass on the SELL copy
     int64_t m = 0, n = 0, nnz = 0;
     double c0 = 0.0;

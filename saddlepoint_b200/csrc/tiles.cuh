@@ -217,6 +217,26 @@ __device__ __forceinline__ void warp_row_sums(const ST *__restrict__ p, int a, i
     for (int q = 0; q < G; ++q) s[q] = ((F32 >> q) & 1u) ? double(warp_sum_down(sf[q])) : warp_sum_down(sd[q]);
 }
 
+// The running sums of a row's G slots, each from -0.0 (slot q in float when bit q of F32 is set).
+template <int G, unsigned F32>
+struct SlotSums {
+    float f[G];
+    double d[G];
+    __device__ __forceinline__ void clear() {
+#pragma unroll
+        for (int q = 0; q < G; ++q) { f[q] = -0.0f; d[q] = -0.0; }
+    }
+    template <class ST>
+    __device__ __forceinline__ void add(const ST (&p)[G]) {
+#pragma unroll
+        for (int q = 0; q < G; ++q) {
+            if ((F32 >> q) & 1u) f[q] += float(p[q]);
+            else d[q] += double(p[q]);
+        }
+    }
+    __device__ __forceinline__ double get(int q) const { return ((F32 >> q) & 1u) ? double(f[q]) : d[q]; }
+};
+
 // Streaming loads of the matrix: each element is read once per pass, so they are
 // hinted to leave L2 first, which keeps the gathered vectors resident there.
 __device__ __forceinline__ int ld_stream(const int *p) { return __ldcs(p); }
