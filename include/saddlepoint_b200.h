@@ -262,8 +262,8 @@ typedef struct {
     int status;
     double objective, dual_objective, primal_residual, dual_residual, gap;
     uint64_t iterations, restarts;
-    int lanes_per_row; /* SpMV variant the tuner chose: 0 = staged tiles (the single-LP passes);
-                          otherwise lane groups, 100 * (lanes per row of A') + (lanes per row of A'ᵀ) */
+    int lanes_per_row; /* SpMV variant: 0 = the single-LP solve's sums (on chip, or staged tiles);
+                          otherwise the tuner's lane groups, 100 * (lanes per row of A') + (lanes per row of A'ᵀ) */
     int handed_off;    /* 1: the instance was still running well after every other instance had
                           been started, and was solved again from the start by the single-LP
                           device solver (sp_solve) */

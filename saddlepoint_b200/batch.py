@@ -37,7 +37,7 @@ class BatchResult:
     gap: float
     iterations: int
     restarts: int
-    lanes_a: int  # lanes per row the tuner picked for A' (0: the staged-tile variant)
+    lanes_a: int  # lanes per row the tuner picked for A' (0: the single-LP solve's sums, on chip or staged tiles)
     lanes_t: int  # ... and for A'ᵀ
     handed_off: bool = False  # finished by the single-LP solver after outrunning its batch budget
 
@@ -47,7 +47,7 @@ class BatchResult:
 
 
 class BatchSolver:
-    """Many LPs solved together by one persistent kernel (one CTA per instance at a time).
+    """Many LPs solved together by persistent kernels (one CTA or small cluster per instance at a time).
 
     ``solve()`` returns one BatchResult per instance and the device time of the launch;
     ``solution(i)`` downloads instance i's x and y in the original space.

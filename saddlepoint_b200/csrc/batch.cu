@@ -2,11 +2,12 @@
 //
 // sp_batch_create packs every LP into one arena (int32 instance-local row
 // pointers, column indices, values, vectors), builds each A'ᵀ on the host with the
-// reference's stable counting sort (problem.rs:88-109, bit for bit), picks the
-// lanes-per-row SpMV variant of every instance with the tuner below, and captures
-// [reset the work counter, launch the persistent kernel] as one CUDA graph.
+// reference's stable counting sort (problem.rs:88-109, bit for bit), plans the instances
+// that run on chip (batch_resident.cuh) in classes by cluster size, picks the SpMV variant
+// of the others with the tuner below, and captures [reset the work counters, launch a
+// persistent kernel per class and one for the others, side by side] as one CUDA graph.
 // sp_batch_solve replays the graph; the scaling, power iteration and PDHG loop of
-// every instance run inside the kernel (batch_kernels.cuh).
+// every instance run inside the kernels.
 #include <algorithm>
 #include <atomic>
 #include <chrono>
@@ -16,7 +17,7 @@
 #include <thread>
 #include <vector>
 
-#include "batch_kernels.cuh"
+#include "batch_resident.cuh"
 #include "internal.cuh"
 
 struct sp_batch {
@@ -29,6 +30,7 @@ struct sp_batch {
     std::vector<void *> bufs;
     cudaGraphExec_t graph = nullptr;
     int grid = 0;
+    int res_clusters[3] = {};  // clusters of each on-chip class
     sp::BatchInst *d_inst = nullptr;
     int *d_counter = nullptr;
     double *av0 = nullptr, *tv0 = nullptr;  // the original values (the kernel scales in place)
@@ -80,7 +82,8 @@ int balloc(sp_batch *b, T **p, int64_t n) {
 // per-iteration time at its size (log nnz) is lowest, with its own L from its mean row
 // lengths. The choice depends on the instance alone, never on the rest
 // of the batch, so an instance is computed the same way alone and in any mix.
-// SP_BATCH_VARIANT=lanes|tiles in the environment forces one variant.
+// SP_BATCH_VARIANT=lanes|tiles in the environment forces one variant. The instances that run
+// on chip (batch_resident.cuh, plan_resident below) are not tuned.
 struct TuneTable {
     bool ready = false;
     int npts = 0;
@@ -92,6 +95,10 @@ static std::mutex g_tune_mu;
 
 int batch_create(sp_ctx *ctx, const sp_lp *lps, int count, const sp_solver_params *params, sp_batch **out,
                  bool tune);
+
+// Work counters of a batch: the tuned kernel's, the on-chip classes', and the instances started.
+constexpr int RES_CLASSES = 3;                      // clusters of 1, 2 and 4 CTAs
+constexpr int BATCH_COUNTERS = 1 + RES_CLASSES + 1;
 
 int calibrate(sp_ctx *ctx, TuneTable *T) {
     // reference LPs: the random LP recipe, m from 60 to 2000, n = 2m, 3-8 nonzeros per column
@@ -119,6 +126,7 @@ int calibrate(sp_ctx *ctx, TuneTable *T) {
         rc = balloc(b, &d_one, 1);
         BatchArgs A2 = b->args;
         A2.count = 1;
+        A2.total = 1;
         A2.order = d_one;
         A2.base.tolerance = 0.0;  // never converged: every run takes exactly its iterations
         A2.handoff_ns = 0;
@@ -134,7 +142,7 @@ int calibrate(sp_ctx *ctx, TuneTable *T) {
                                         cudaMemcpyDeviceToDevice, st));
             SP_CUDA_TRY(cudaMemcpyAsync(b->args.t_v + I.nz, b->tv0 + I.nz, sizeof(double) * I.nnz,
                                         cudaMemcpyDeviceToDevice, st));
-            SP_CUDA_TRY(cudaMemsetAsync(b->d_counter, 0, sizeof(int), st));
+            SP_CUDA_TRY(cudaMemsetAsync(b->d_counter, 0, BATCH_COUNTERS * sizeof(int), st));
             SP_CUDA_TRY(cudaEventRecord(e0, st));
             k_batch<NT><<<1, NT, b->smem, st>>>(A2);
             SP_CUDA_TRY(cudaEventRecord(e1, st));
@@ -168,6 +176,9 @@ int tune_variants(sp_batch *b) {
     int forced = -1;
     if (const char *env = getenv("SP_BATCH_VARIANT"))
         forced = !strcmp(env, "lanes") ? VARIANT_LANES : (!strcmp(env, "tiles") ? VARIANT_TILES : -1);
+    bool all = true;  // every instance runs on chip: there is nothing to tune
+    for (const BatchInst &I : inst) all = all && I.variant == VARIANT_RES;
+    if (all) return SP_OK;
     if (forced < 0) {
         const int dev = b->ctx->device;
         std::lock_guard<std::mutex> lock(g_tune_mu);
@@ -193,6 +204,7 @@ int tune_variants(sp_batch *b) {
             return T.us[v][p] + f * (T.us[v][p + 1] - T.us[v][p]);
         };
         for (auto &I : inst) {
+            if (I.variant == VARIANT_RES) continue;
             int best = 0;
             for (int v = 1; v < TUNE_SHAPES; ++v)
                 if (estimate(v, I.nnz) < estimate(best, I.nnz)) best = v;
@@ -206,6 +218,206 @@ int tune_variants(sp_batch *b) {
     SP_CUDA_TRY(cudaStreamSynchronize(st));
     return SP_OK;
 }
+
+// ------------------------------------------------------------------ instances on chip
+
+constexpr int RES_BATCH_SMEM = (int)STREAM_SMEM_MAX - 4096;  // dynamic shared memory, beside ResShared
+
+// The plans of the instances that run on chip, by class (clusters of 1 << class CTAs).
+struct ResBatchPlan {
+    std::vector<ResBatchInst> inst;           // by instance; id = -1: not on chip
+    std::vector<int> cls;
+    std::vector<ResPlan> a, t;
+};
+
+// Which instances run on chip, and how: the smallest cluster whose CTAs hold the instance's
+// rows and columns (clusters cost throughput: four CTAs take a 1,900 x 3,800 LP 4.3 µs an
+// iteration, one takes a 400 x 800 LP 2.9 µs); not those with a row longer than a tile, and
+// none when another variant is forced. An instance's choice depends on it alone. Measured on
+// 1,024 LPs of 50-2,000 rows, 640 iterations each with set-up (B200): 202 ms with the tuned
+// variants, 36 ms on chip.
+ResBatchPlan plan_resident(sp_batch *b, const std::vector<int> &arp, const std::vector<int> &trp) {
+    ResBatchPlan P;
+    const int count = b->count;
+    if (const char *env = getenv("SP_BATCH_VARIANT"))
+        if (!strcmp(env, "lanes") || !strcmp(env, "tiles")) return P;
+    P.inst.resize(count);
+    P.cls.assign(count, -1);
+    P.a.resize(count);
+    P.t.resize(count);
+    auto run = [&](int i0, int i1) {
+        for (int i = i0; i < i1; ++i) {
+            const BatchInst &I = b->inst[i];
+            ResBatchInst &q = P.inst[i];
+            q = ResBatchInst{};
+            q.id = -1;
+            if (I.m < 1 || I.n < 1) continue;
+            const int *ra = arp.data() + I.rpa, *rt = trp.data() + I.rpt;
+            int longest = 0;
+            for (int r = 0; r < I.m; ++r) longest = std::max(longest, ra[r + 1] - ra[r]);
+            for (int r = 0; r < I.n; ++r) longest = std::max(longest, rt[r + 1] - rt[r]);
+            if (longest > TILE_NNZ) continue;
+            for (int k = 0; k < RES_CLASSES; ++k) {
+                const int nc = 1 << k;
+                if (I.m > nc * RES_BATCH_PA || I.n > nc * RES_BATCH_PT) continue;
+                ResPlan &A = P.a[i], &T = P.t[i];
+                A = ResPlan{};
+                T = ResPlan{};
+                res_plan(ra, I.m, nc, &A);
+                res_plan(rt, I.n, nc, &T);
+                if (A.most_rows > RES_BATCH_PA || T.most_rows > RES_BATCH_PT) continue;
+                auto bytes = [&](bool es) {
+                    return ResBatchPlaces(I.m, I.n, b->mixed, A.most_tasks, T.most_tasks, A.most_slots, T.most_slots, es, 8)
+                        .total;
+                };
+                if (bytes(false) > RES_BATCH_SMEM) continue;
+                q.id = i;
+                q.es = bytes(true) <= RES_BATCH_SMEM;
+                q.heavyA = A.heavy;
+                q.heavyT = T.heavy;
+                const int ma[] = {A.most_rows, A.most_slots, A.most_tasks}, mt[] = {T.most_rows, T.most_slots, T.most_tasks};
+                std::copy(ma, ma + 3, q.mostA);
+                std::copy(mt, mt + 3, q.mostT);
+                std::copy(A.p0.begin(), A.p0.end(), q.pA);
+                std::copy(A.s0.begin(), A.s0.end(), q.sA);
+                std::copy(T.p0.begin(), T.p0.end(), q.pT);
+                std::copy(T.s0.begin(), T.s0.end(), q.sT);
+                P.cls[i] = k;
+                break;
+            }
+        }
+    };
+    const int nt = std::max(1, std::min<int>({16, (int)std::thread::hardware_concurrency(), count}));
+    std::vector<std::thread> th;
+    for (int t = 0; t < nt; ++t) th.emplace_back(run, (int)((int64_t)count * t / nt), (int)((int64_t)count * (t + 1) / nt));
+    for (auto &t : th) t.join();
+    for (int i = 0; i < count; ++i)
+        if (P.inst[i].id >= 0) b->inst[i].variant = VARIANT_RES;
+    return P;
+}
+
+template <int NC>
+const void *res_batch_kernel(bool mixed) {
+    return mixed ? (const void *)k_batch_res<NC, true> : (const void *)k_batch_res<NC, false>;
+}
+const void *res_batch_kernel(int cls, bool mixed) {
+    return cls == 0 ? res_batch_kernel<1>(mixed) : cls == 1 ? res_batch_kernel<2>(mixed) : res_batch_kernel<4>(mixed);
+}
+
+// The launch of a class: its clusters, one CTA to an SM.
+int resident_config(sp_batch *b, int cls, unsigned clusters, cudaStream_t st, cudaLaunchConfig_t *cfg,
+                    cudaLaunchAttribute *at) {
+    *cfg = cudaLaunchConfig_t{};
+    cfg->gridDim = dim3(clusters << cls);
+    cfg->blockDim = dim3(RES_BT);
+    cfg->dynamicSmemBytes = RES_BATCH_SMEM;
+    cfg->stream = st;
+    at->id = cudaLaunchAttributeClusterDimension;
+    at->val.clusterDim.x = 1u << cls;
+    at->val.clusterDim.y = 1;
+    at->val.clusterDim.z = 1;
+    if (cls) {
+        cfg->attrs = at;
+        cfg->numAttrs = 1;
+    }
+    SP_CUDA_TRY(cudaFuncSetAttribute(res_batch_kernel(cls, b->mixed), cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     RES_BATCH_SMEM));
+    return SP_OK;
+}
+
+// Uploads the plans; fills R and the classes (largest instances first, as `order` has them).
+int upload_resident(sp_batch *b, const ResBatchPlan &P, const std::vector<int> &order, BatchRes *R,
+                    ResBatchClass *classes) {
+    if (P.inst.empty()) return SP_OK;
+    std::vector<uint16_t> pa(b->total_m), pt(b->total_n), ia(b->total_m), it(b->total_n);
+    std::vector<ResTask> tasks;
+    std::vector<int> wt;
+    std::vector<ResBatchInst> cls[RES_CLASSES];
+    size_t scratch[RES_CLASSES] = {};
+    for (int i : order) {
+        if (P.cls[i] < 0) continue;
+        const BatchInst &I = b->inst[i];
+        ResBatchInst q = P.inst[i];
+        const ResPlan &A = P.a[i], &T = P.t[i];
+        std::copy(A.perm.begin(), A.perm.end(), pa.begin() + I.mo);
+        std::copy(A.inv.begin(), A.inv.end(), ia.begin() + I.mo);
+        std::copy(T.perm.begin(), T.perm.end(), pt.begin() + I.no);
+        std::copy(T.inv.begin(), T.inv.end(), it.begin() + I.no);
+        q.tasksA = (long long)tasks.size();
+        tasks.insert(tasks.end(), A.tasks.begin(), A.tasks.end());
+        q.tasksT = (long long)tasks.size();
+        tasks.insert(tasks.end(), T.tasks.begin(), T.tasks.end());
+        q.wtA = (int)wt.size();
+        wt.insert(wt.end(), A.wt.begin(), A.wt.end());
+        q.wtT = (int)wt.size();
+        wt.insert(wt.end(), T.wt.begin(), T.wt.end());
+        const int k = P.cls[i];
+        cls[k].push_back(q);
+        scratch[k] = std::max(scratch[k], ResScratch(A.slots, T.slots, I.m, I.n, I.nta, I.ntt, b->mixed).total);
+    }
+    cudaStream_t st = b->ctx->stream;
+    int rc;
+    auto put = [&](const auto &h, auto **d) -> int {
+        using V = std::remove_reference_t<decltype(h[0])>;
+        std::remove_const_t<V> *p = nullptr;
+        if (int e = balloc(b, &p, (int64_t)h.size())) return e;
+        if (!h.empty()) SP_CUDA_TRY(cudaMemcpyAsync(p, h.data(), sizeof(V) * h.size(), cudaMemcpyHostToDevice, st));
+        *d = p;
+        return SP_OK;
+    };
+    if ((rc = put(pa, &R->permA)) || (rc = put(pt, &R->permT)) || (rc = put(ia, &R->invA)) || (rc = put(it, &R->invT)) ||
+        (rc = put(tasks, &R->tasks)) || (rc = put(wt, &R->wt)))
+        return rc;
+    for (int k = 0; k < RES_CLASSES; ++k) {
+        ResBatchClass &c = classes[k];
+        c.count = (int)cls[k].size();
+        if (!c.count) continue;
+        if ((rc = put(cls[k], &c.inst))) return rc;
+        cudaLaunchConfig_t cfg;
+        cudaLaunchAttribute at;
+        if ((rc = resident_config(b, k, 1, st, &cfg, &at))) return rc;
+        int most = 0;
+        if (k) SP_CUDA_TRY(cudaOccupancyMaxActiveClusters(&most, res_batch_kernel(k, b->mixed), &cfg));
+        else most = b->ctx->sms;
+        b->res_clusters[k] = std::max(1, std::min(c.count, most));
+        c.counter = b->args.counter + 1 + k;
+        c.scratch_bytes = scratch[k];
+        if ((rc = balloc(b, &c.scratch, (int64_t)scratch[k] * b->res_clusters[k]))) return rc;
+    }
+    SP_CUDA_TRY(cudaStreamSynchronize(st));  // the host's copies end here
+    return SP_OK;
+}
+
+int launch_resident(sp_batch *b, const BatchRes &R, const ResBatchClass &c, int cls, cudaStream_t st) {
+    cudaLaunchConfig_t cfg;
+    cudaLaunchAttribute at;
+    int rc = resident_config(b, cls, (unsigned)b->res_clusters[cls], st, &cfg, &at);
+    if (rc) return rc;
+    void *args[] = {(void *)&b->args, (void *)&R, (void *)&c};
+    SP_CUDA_TRY(cudaLaunchKernelExC(&cfg, res_batch_kernel(cls, b->mixed), args));
+    return SP_OK;
+}
+
+// Streams and events that shape the batch's graph while it is captured.
+struct SideStreams {
+    cudaStream_t st[RES_CLASSES] = {};
+    cudaEvent_t fork = nullptr, done[RES_CLASSES] = {};
+    int init() {
+        SP_CUDA_TRY(cudaEventCreateWithFlags(&fork, cudaEventDisableTiming));
+        for (int k = 0; k < RES_CLASSES; ++k) {
+            SP_CUDA_TRY(cudaStreamCreateWithFlags(&st[k], cudaStreamNonBlocking));
+            SP_CUDA_TRY(cudaEventCreateWithFlags(&done[k], cudaEventDisableTiming));
+        }
+        return SP_OK;
+    }
+    ~SideStreams() {
+        for (cudaStream_t x : st)
+            if (x) cudaStreamDestroy(x);
+        for (cudaEvent_t x : done)
+            if (x) cudaEventDestroy(x);
+        if (fork) cudaEventDestroy(fork);
+    }
+};
 
 // The instance as an sp_lp again, from the arena's original data on the device.
 struct HostLp {
@@ -483,18 +695,25 @@ int batch_create(sp_ctx *ctx, const sp_lp *lps, int count, const sp_solver_param
         std::copy(tiles_a[i].begin(), tiles_a[i].end(), h_ta.begin() + b->inst[i].ta);
         std::copy(tiles_t[i].begin(), tiles_t[i].end(), h_tt.begin() + b->inst[i].tt);
     }
+    // the instances on chip; the others are the tuned kernel's
+    ResBatchPlan onchip;
+    if (tune) onchip = plan_resident(b, h_arp, h_trp);
     // processing order: largest first, so the long instances start early
-    std::vector<int> order(count);
-    std::iota(order.begin(), order.end(), 0);
-    std::stable_sort(order.begin(), order.end(), [&](int a, int c) { return b->inst[a].nnz > b->inst[c].nnz; });
+    std::vector<int> all(count), order;
+    std::iota(all.begin(), all.end(), 0);
+    std::stable_sort(all.begin(), all.end(), [&](int a, int c) { return b->inst[a].nnz > b->inst[c].nnz; });
+    for (int i : all)
+        if (b->inst[i].variant != VARIANT_RES) order.push_back(i);
 
     BatchArgs &A = b->args;
-    A.count = count;
+    A.count = (int)order.size();
+    A.total = count;
     A.mixed = b->mixed;
     BatchInst *d_inst;
     int *d_order, *d_counter, *arp, *aci, *trp, *tci;
     double *av, *tv, *oc, *olv, *ouv, *olc, *ouc;
-    if ((rc = balloc(b, &d_inst, count)) || (rc = balloc(b, &d_order, count)) || (rc = balloc(b, &d_counter, 1)) ||
+    if ((rc = balloc(b, &d_inst, count)) || (rc = balloc(b, &d_order, count)) ||
+        (rc = balloc(b, &d_counter, BATCH_COUNTERS)) ||
         (rc = balloc(b, &arp, rpa)) || (rc = balloc(b, &trp, rpt)) || (rc = balloc(b, &aci, nz)) ||
         (rc = balloc(b, &tci, nz)) || (rc = balloc(b, &av, nz)) || (rc = balloc(b, &tv, nz)) ||
         (rc = balloc(b, &oc, no)) || (rc = balloc(b, &olv, no)) || (rc = balloc(b, &ouv, no)) ||
@@ -506,7 +725,7 @@ int batch_create(sp_ctx *ctx, const sp_lp *lps, int count, const sp_solver_param
         return SP_OK;
     };
     if ((rc = up(d_inst, b->inst.data(), sizeof(BatchInst) * count)) ||
-        (rc = up(d_order, order.data(), sizeof(int) * count)) || (rc = up(arp, h_arp.data(), sizeof(int) * rpa)) ||
+        (rc = up(d_order, order.data(), sizeof(int) * order.size())) || (rc = up(arp, h_arp.data(), sizeof(int) * rpa)) ||
         (rc = up(trp, h_trp.data(), sizeof(int) * rpt)) || (rc = up(aci, h_aci.data(), sizeof(int) * nz)) ||
         (rc = up(tci, h_tci.data(), sizeof(int) * nz)) || (rc = up(av, h_av.data(), sizeof(double) * nz)) ||
         (rc = up(tv, h_tv.data(), sizeof(double) * nz)) || (rc = up(oc, h_c.data(), sizeof(double) * no)) ||
@@ -521,6 +740,9 @@ int batch_create(sp_ctx *ctx, const sp_lp *lps, int count, const sp_solver_param
     A.inst = d_inst;
     A.order = d_order;
     A.counter = d_counter;
+    A.started = d_counter + 1 + RES_CLASSES;
+    A.av0 = av0;
+    A.tv0 = tv0;
     A.a_rp = arp;
     A.a_ci = aci;
     A.t_rp = trp;
@@ -589,23 +811,45 @@ int batch_create(sp_ctx *ctx, const sp_lp *lps, int count, const sp_solver_param
     SP_CUDA_TRY(cudaFuncSetAttribute((const void *)k_batch<NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     int per_sm = 0;
     SP_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_batch<NT>, NT, smem));
-    b->grid = std::max(1, std::min(count, std::max(1, per_sm) * ctx->sms));
+    b->grid = std::max(1, std::min(A.count, std::max(1, per_sm) * ctx->sms));
     b->d_inst = d_inst;
     b->d_counter = d_counter;
     b->av0 = av0;
     b->tv0 = tv0;
     b->smem = smem;
     if (tune && (rc = tune_variants(b))) return bail(rc, "sp_batch_create: tuner");
-    // one graph: restore the original values, reset the counter, run the persistent kernel
+    BatchRes R{};
+    ResBatchClass classes[RES_CLASSES] = {};
+    if ((rc = upload_resident(b, onchip, all, &R, classes))) return bail(rc, "sp_batch_create: on-chip plans");
+    // one graph: reset the counters, then the on-chip classes (the largest instances first) and,
+    // where instances are left to it, the tuned kernel on values restored as given, side by side
     cudaGraph_t g;
     SP_CUDA_TRY(cudaStreamSynchronize(st));
+    SideStreams side;
+    if ((rc = side.init())) return bail(rc, "sp_batch_create: streams");
     SP_CUDA_TRY(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
-    cudaMemcpyAsync(av, av0, sizeof(double) * nz, cudaMemcpyDeviceToDevice, st);
-    cudaMemcpyAsync(tv, tv0, sizeof(double) * nz, cudaMemcpyDeviceToDevice, st);
-    cudaMemsetAsync(d_counter, 0, sizeof(int), st);
+    cudaMemsetAsync(d_counter, 0, BATCH_COUNTERS * sizeof(int), st);
     cudaMemsetAsync(A.drain_ns, 0, sizeof(unsigned long long), st);
-    k_batch<NT><<<b->grid, NT, smem, st>>>(A);
+    cudaEventRecord(side.fork, st);
+    int launch_rc = SP_OK;
+    for (int k = RES_CLASSES - 1; k >= 0; --k) {
+        if (classes[k].count == 0) continue;
+        cudaStreamWaitEvent(side.st[k], side.fork, 0);
+        if (!launch_rc) launch_rc = launch_resident(b, R, classes[k], k, side.st[k]);
+        cudaEventRecord(side.done[k], side.st[k]);
+    }
+    if (A.count > 0) {
+        cudaMemcpyAsync(av, av0, sizeof(double) * nz, cudaMemcpyDeviceToDevice, st);
+        cudaMemcpyAsync(tv, tv0, sizeof(double) * nz, cudaMemcpyDeviceToDevice, st);
+        k_batch<NT><<<b->grid, NT, smem, st>>>(A);
+    }
+    for (int k = 0; k < RES_CLASSES; ++k)
+        if (classes[k].count) cudaStreamWaitEvent(st, side.done[k], 0);
     SP_CUDA_TRY(cudaStreamEndCapture(st, &g));
+    if (launch_rc) {
+        cudaGraphDestroy(g);
+        return bail(launch_rc, "sp_batch_create: on-chip launch");
+    }
     cudaError_t e = cudaGraphInstantiate(&b->graph, g, 0);
     cudaGraphDestroy(g);
     if (e != cudaSuccess) return bail(SP_ERR_CUDA, std::string("graph: ") + cudaGetErrorString(e));

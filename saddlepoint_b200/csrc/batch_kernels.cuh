@@ -34,20 +34,22 @@ struct BatchInst {
     int maximize, pad2;
 };
 
-enum : int { VARIANT_LANES = 0, VARIANT_TILES = 1 };
+enum : int { VARIANT_LANES = 0, VARIANT_TILES = 1, VARIANT_RES = 2 };  // RES: on chip (batch_resident.cuh)
 
 struct BatchArgs {
     const BatchInst *inst;
     const int *order;  // processing order (largest first)
-    int count;
+    int count;           // ... of this kernel's instances
     int *counter;
-    // The tail hand-off: once every instance has been claimed (drain_ns: when, 0 before),
-    // an instance still running handoff_ns later stops at its next check and is
-    // finished by the single-LP solver on the host's side (0: never).
+    int *started, total; // instances that any kernel of the batch has started, and all of them
+    // The tail hand-off: once every instance has been claimed (drain_ns: when a CTA found
+    // none left, 0 before), an instance still running handoff_ns later stops at its next
+    // check and is finished by the single-LP solver on the host's side (0: never).
     unsigned long long *drain_ns;
     unsigned long long handoff_ns;
     const int *a_rp, *a_ci, *t_rp, *t_ci;
     double *a_v, *t_v;
+    const double *av0, *tv0;  // the values as given
     float *a_v32, *t_v32;
     const double *oc, *olc, *ouc, *olv, *ouv;  // original vectors
     double *c, *lc, *uc, *lv, *uv, *pf, *df, *rs, *cs;
@@ -65,16 +67,29 @@ struct BatchArgs {
     int mixed;
 };
 
-// Thread 0, after a check that did not end the solve: stop for the hand-off when the
-// queue drained more than handoff_ns ago (the instance is a straggler of the tail).
-__device__ __forceinline__ void tail_handoff(const BatchArgs &A, DevState &st) {
-    if (st.done || A.handoff_ns == 0) return;
+// Whether the queue drained more than handoff_ns ago: an instance still running is then a
+// straggler of the tail.
+__device__ __forceinline__ bool tail_due(const BatchArgs &A) {
+    if (A.handoff_ns == 0) return false;
     const unsigned long long drained = *reinterpret_cast<volatile unsigned long long *>(A.drain_ns);
-    if (drained && global_ns() - drained > A.handoff_ns) {
+    return drained && global_ns() - drained > A.handoff_ns;
+}
+
+// Thread 0, after a check that did not end the solve: stop for the hand-off where it is due.
+__device__ __forceinline__ void tail_handoff(const BatchArgs &A, DevState &st) {
+    if (!st.done && tail_due(A)) {
         st.done = 1;
         st.status = SP_STATUS_ITERATION_LIMIT;
         st.handoff = 1;
     }
+}
+
+// One thread: the next of `count` instances from a kernel's counter (count or more: none left).
+__device__ __forceinline__ int batch_claim(const BatchArgs &A, int *counter, int count) {
+    const int slot = atomicAdd(counter, 1);
+    if (slot < count) atomicAdd(A.started, 1);
+    else if (atomicAdd(A.started, 0) == A.total) atomicCAS(A.drain_ns, 0ull, global_ns());
+    return slot;
 }
 
 template <int BT, int K>
@@ -820,14 +835,11 @@ __global__ void __launch_bounds__(BT) k_batch(BatchArgs A) {
     __shared__ double bc[8];
     __shared__ int next;
     for (;;) {
-        if (threadIdx.x == 0) next = atomicAdd(A.counter, 1);
+        if (threadIdx.x == 0) next = batch_claim(A, A.counter, A.count);
         __syncthreads();
         const int slot = next;
         __syncthreads();
-        if (slot >= A.count) {
-            if (threadIdx.x == 0) atomicCAS(A.drain_ns, 0ull, global_ns());
-            return;
-        }
+        if (slot >= A.count) return;
         batch_solve_one<BT>(A, A.order[slot], sh, st, prm, bc, dsm);
     }
 }

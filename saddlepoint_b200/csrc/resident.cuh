@@ -204,8 +204,9 @@ struct ResPlaces {
     static constexpr int YA = 40 * PT, LC = YA + 8 * PA, UC = YA + 16 * PA, END = YA + 24 * PA;
     int y, xbar, y32, xbar32, tasksA, tasksT, wtA, wtT, valA, valT, atA, atT, total;
     __host__ __device__ static int up(int b) { return (b + 15) & ~15; }
-    // tasks and slots: the most of one CTA (A', A'ᵀ); entries: with entries in shared memory
-    __host__ __device__ ResPlaces(int m, int n, bool lo, int ta, int tt, int sa, int st, bool entries) {
+    // lo: with the FP32 vectors; tasks and slots: the most of one CTA (A', A'ᵀ); entries: with
+    // entries of vb bytes a value in shared memory
+    __host__ __device__ ResPlaces(int m, int n, bool lo, int ta, int tt, int sa, int st, bool entries, int vb) {
         int at = END;
         auto take = [&](int bytes) {
             const int a = at;
@@ -220,7 +221,6 @@ struct ResPlaces {
         tasksT = take((int)sizeof(ResTask) * tt);
         wtA = take(4 * (RES_W + 1));
         wtT = take(4 * (RES_W + 1));
-        const int vb = lo ? 4 : 8;
         valA = entries ? take(vb * sa) : 0;
         valT = entries ? take(vb * st) : 0;
         atA = entries ? take(2 * sa) : 0;
@@ -283,6 +283,7 @@ struct ResShared {
     long long trace_cap;
     int mixed;
     int count_bad_first;        // a non-finite first iteration counts (the batch's rule)
+    float stop;                 // 1: the batch's hand-off is due (every CTA's copy, by rank 0)
     double sh[RES_GROUPS * NP_P * (NT / 32) + NP_P];
     double wtab[RES_WTAB];
 };
@@ -955,12 +956,17 @@ __device__ __noinline__ void res_first(ResShared &sh) {
 
 // The check iteration that ends an epoch of E iterations: its passes, the decisions (every CTA
 // takes the same ones from the same sums, on its own copy of the state), and the Halpern step
-// or the restart's copies. `stop` is called by thread 0 between the two (the batch's hand-off).
+// or the restart's copies. `stop` says whether an unfinished solve stops here for the batch's
+// hand-off: one CTA asks it, so that all of them agree.
 template <bool CL, bool LO, class Stop>
 __device__ __noinline__ void res_check(ResShared &sh, unsigned long long E, Stop stop) {
     const ResCtx &R = sh.R;
     const SolverPtrs &S = R.S;
     DevState *st = &sh.st;
+    if (threadIdx.x == 0 && (!CL || cluster_rank() == 0)) {
+        sh.stop = stop() ? 1.0f : 0.0f;
+        publish<CL>(&sh.stop);
+    }
     {
         const IterScalars sc = res_scalars(sh, 0.0);
         res_primal<CL, LO, 2>(R, sc);
@@ -990,7 +996,11 @@ __device__ __noinline__ void res_check(ResShared &sh, unsigned long long E, Stop
                 if ((long long)st->checks - 1 < sh.trace_cap) sh.trace[st->checks - 1] = rec;
             st->trace_len = st->checks;
         }
-        stop(*st);
+        if (!st->done && sh.stop != 0.0f) {
+            st->done = 1;
+            st->status = SP_STATUS_ITERATION_LIMIT;
+            st->handoff = 1;
+        }
     }
     __syncthreads();
     if (st->done) return;
@@ -1022,7 +1032,7 @@ template <int NC, bool LO, bool ES, int PT, int PA, class Stop>
 __device__ __forceinline__ void res_epochs(ResShared &sh, const ResPlaces<PT, PA> &L, Stop stop) {
     constexpr bool CL = NC > 1;
     while (!sh.st.done && sh.st.total < sh.until && LO == (sh.mixed && !sh.st.fp64)) {
-        unsigned long long E = sh.prm.max_iterations - sh.st.total;
+        unsigned long long E = sh.prm.max_iterations > sh.st.total ? sh.prm.max_iterations - sh.st.total : 1;
         if (sh.prm.check_every && sh.prm.check_every < E) E = sh.prm.check_every;
         const bool first = sh.st.k == 0 && E > 1;
         if (first) {
@@ -1140,11 +1150,12 @@ struct ResArgs {
 };
 
 __host__ __device__ inline ResSolverPlaces res_solver_places(const ResSrc &A, const ResSrc &T, bool lo, bool entries) {
-    return ResSolverPlaces(A.rows, T.rows, lo, A.most_tasks, T.most_tasks, A.most_slots, T.most_slots, entries);
+    return ResSolverPlaces(A.rows, T.rows, lo, A.most_tasks, T.most_tasks, A.most_slots, T.most_slots, entries,
+                           lo ? 4 : 8);
 }
 
 struct ResNoStop {
-    __device__ void operator()(DevState &) const {}
+    __device__ bool operator()() const { return false; }
 };
 
 // Epochs of the solver's state in one precision until its total is `until`. In the mixed

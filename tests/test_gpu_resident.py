@@ -108,3 +108,45 @@ def test_resident_nonfinite_iterates_are_a_numerical_error(gpu_backend):
         with pytest.raises(sp().SolveError) as e:
             solve_with(engine, lp, p, gpu_backend)
         assert e.value.code == 5
+
+
+@pytest.mark.parametrize("mixed", [False, True])
+@pytest.mark.parametrize("kw", [dict(max_iterations=300), dict(max_iterations=90, check_every=0),
+                                dict(max_iterations=100, check_every=7)])
+def test_batch_on_chip_equals_the_solo_solve(kw, mixed, gpu_backend):
+    """Instances at the edges of the classes (clusters of 1, 2 and 4 CTAs), with warp rows, and
+    one beyond them beside: each has the solo solve's bits, twice."""
+    ms = [9, 60, 300, 512, 513, 1024, 1025, 2000, 2048]
+    lps = [sp().generate_random_lp(40 + m, m, 2 * m, (3, 8)) for m in ms]
+    lps += [sp().generate_random_lp(7, 8, 1, (3, 3)), sp().generate_transport_lp(9, 40, 60), netlib_lp("25fv47"),
+            netlib_lp("israel")]
+    beyond = sp().generate_random_lp(8, 2100, 4200, (3, 8))
+    p = sp().SolverParams(tolerance=0.0, infeasibility_tolerance=0.0,
+                          precision=sp().Precision.Mixed if mixed else sp().Precision.FP64, **kw)
+    b = sp().BatchSolver(lps + [beyond], p, gpu_backend)
+    for _ in range(2):
+        res, _ = b.solve()
+        for i, lp in enumerate(lps):
+            solo = sp().solve(lp, p, gpu_backend)
+            x, y = b.solution(i)
+            assert res[i].variant == "tiles" and not res[i].handed_off
+            assert res[i].iterations == solo.iterations and res[i].restarts == solo.restarts, lp.name
+            assert res[i].objective == solo.objective and res[i].status == int(solo.status), lp.name
+            assert np.array_equal(x, solo.x) and np.array_equal(y, solo.y), lp.name
+        assert res[len(lps)].iterations == kw["max_iterations"]
+
+
+def test_batch_hand_off_from_a_cluster(gpu_backend, monkeypatch):
+    """Stragglers on clusters stop at a check that all of the cluster's CTAs agree on, and get
+    the solo solve's result."""
+    monkeypatch.setenv("SP_BATCH_HANDOFF_S", "1e-9")
+    lps = [sp().generate_random_lp(60 + m, m, 2 * m, (3, 8)) for m in (700, 900, 1500, 1900)]
+    p = params(1000)
+    b = sp().BatchSolver(lps, p, gpu_backend)
+    res, _ = b.solve()
+    assert sum(r.handed_off for r in res) >= len(lps) - 1
+    for i, lp in enumerate(lps):
+        solo = sp().solve(lp, p, gpu_backend)
+        x, y = b.solution(i)
+        assert res[i].iterations == solo.iterations == 1000 and res[i].objective == solo.objective
+        assert np.array_equal(x, solo.x) and np.array_equal(y, solo.y)
