@@ -150,3 +150,22 @@ def test_batch_hand_off_from_a_cluster(gpu_backend, monkeypatch):
         x, y = b.solution(i)
         assert res[i].iterations == solo.iterations == 1000 and res[i].objective == solo.objective
         assert np.array_equal(x, solo.x) and np.array_equal(y, solo.y)
+
+
+def test_batch_solutions_in_any_order(gpu_backend):
+    """Solutions fetched in order (a block ahead), out of order, twice, and after another solve
+    are the same; an instance larger than a block is fetched by itself."""
+    ms = [40, 2000, 9, 300, 25000, 700, 60, 2048, 80]
+    lps = [sp().generate_random_lp(80 + i, m, 2 * m, (2, 4)) for i, m in enumerate(ms)]
+    b = sp().BatchSolver(lps, params(40), gpu_backend)
+    b.solve()
+    ahead = [b.solution(i) for i in range(len(ms))]
+    for i in (8, 3, 3, 4, 5, 6, 0, 1, 7, 2):
+        x, y = b.solution(i)
+        assert np.array_equal(x, ahead[i][0]) and np.array_equal(y, ahead[i][1])
+    solo = sp().solve(lps[1], params(40), gpu_backend)
+    assert np.array_equal(ahead[1][0], solo.x) and np.array_equal(ahead[1][1], solo.y)
+    b.solve()
+    for i in range(len(ms)):
+        x, y = b.solution(i)
+        assert len(x) == 2 * ms[i] and np.array_equal(x, ahead[i][0]) and np.array_equal(y, ahead[i][1])
