@@ -22,7 +22,7 @@ ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 FLAGS = ["-std=c++17", "-O3", "-lineinfo", "--fmad=false", "-Xcompiler", "-fPIC,-O3", "-Xptxas", "-O3"]
 CU = ["backend.cu", "solver.cu", "batch.cu", "serve.cu", "noalloc.cu", "triplets.cu"]
 CPP = ["host.cpp", "mps.cpp", "presolve.cpp", "polish.cpp"]
-HEADERS = ["common.cuh", "internal.cuh", "tiles.cuh", "stream.cuh", "sell.cuh", "control.cuh", "solver_kernels.cuh", "resident.cuh", "solver_state.h", "batch_kernels.cuh", "batch_resident.cuh"]
+HEADERS = ["common.cuh", "internal.cuh", "tiles.cuh", "stream.cuh", "sell.cuh", "control.cuh", "solver_kernels.cuh", "resident.cuh", "grid.cuh", "solver_state.h", "batch_kernels.cuh", "batch_resident.cuh"]
 
 
 def _sources():

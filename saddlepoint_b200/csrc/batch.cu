@@ -268,8 +268,8 @@ ResBatchPlan plan_resident(sp_batch *b, const std::vector<int> &arp, const std::
                 ResPlan &A = P.a[i], &T = P.t[i];
                 A = ResPlan{};
                 T = ResPlan{};
-                res_plan(ra, I.m, nc, &A);
-                res_plan(rt, I.n, nc, &T);
+                res_plan(ra, I.m, nc, true, &A);
+                res_plan(rt, I.n, nc, true, &T);
                 if (A.most_rows > RES_BATCH_PA || T.most_rows > RES_BATCH_PT) continue;
                 auto bytes = [&](bool es) {
                     return ResBatchPlaces(I.m, I.n, b->mixed, A.most_tasks, T.most_tasks, A.most_slots, T.most_slots, es, 8)
@@ -493,6 +493,7 @@ int hand_off(sp_batch *b, std::vector<sp_batch_result> &res) {
     auto work = [&]() {
         sp_ctx *ctx = nullptr;
         int rc = sp_ctx_create(b->ctx->device, &ctx);
+        if (!rc) ctx->shared = true;
         size_t k;
         while (!rc && (k = next.fetch_add(1)) < todo.size()) {
             const int i = todo[k];

@@ -69,7 +69,7 @@ struct ResScratch {
 // Calls f(position, first slot, slot step, slots) for each row of this warp, lane by lane:
 // the slots of a slice's row are 32 apart, those of a warp row consecutive; both end in padding.
 template <class F>
-__device__ __forceinline__ void res_rows(const ResSide &M, const F &f) {
+__device__ __forceinline__ void res_rows(const ResSide<uint16_t> &M, const F &f) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int t1 = (&dsm_at<int>(M.wt))[warp + 1];
 #pragma unroll 1
@@ -82,7 +82,7 @@ __device__ __forceinline__ void res_rows(const ResSide &M, const F &f) {
 }
 
 // This CTA's slots from the instance's CSR arrays (k_res_fill's layout).
-__device__ __forceinline__ void res_fill(const ResSide &M, uint16_t *ci_out, double *v_out, const int *rp, const int *ci,
+__device__ __forceinline__ void res_fill(const ResSide<uint16_t> &M, uint16_t *ci_out, double *v_out, const int *rp, const int *ci,
                                          const double *v, const uint16_t *other_inv, int other_rows) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int t1 = (&dsm_at<int>(M.wt))[warp + 1];
@@ -119,10 +119,10 @@ __device__ __forceinline__ double factor_of(double v) { return (v > 0.0 && isfin
 // columns. Row factors go through y and column factors through x̄ (whole in every CTA, the
 // padding's 1.0 behind them); new factors wait in xn and yn (this CTA's positions) while the
 // old ones are read. rs, cs: the products of all factors, over positions.
-template <bool CL>
-__device__ __noinline__ void res_scale(ResShared &sh, const BatchArgs &A, double *vA, double *vT, double *rs, double *cs) {
-    const ResCtx &R = sh.R;
-    const ResSide &MA = R.A, &MT = R.T;
+template <int NC>
+__device__ __noinline__ void res_scale(ResShared<uint16_t> &sh, const BatchArgs &A, double *vA, double *vT, double *rs, double *cs) {
+    const ResCtx<uint16_t> &R = sh.R;
+    const ResSide<uint16_t> &MA = R.A, &MT = R.T;
     double *fr = R.S.y, *fc = R.S.xbar, *yn = R.S.ya, *xn = R.S.xa;
     const int noneA = MT.rows, noneT = MA.rows;  // the padding's columns
     auto span = [](const uint16_t *ci, const double *v, int none, int o, int step, int n, double &lo, double &hi) {
@@ -141,11 +141,11 @@ __device__ __noinline__ void res_scale(ResShared &sh, const BatchArgs &A, double
             double lo = INFINITY, hi = 0.0;
             span(MA.ci, vA, noneA, o, step, n, lo, hi);
             fr[k] = factor_geo(lo, hi);
-            publish<CL>(fr + k);
+            publish<NC>(fr + k);
         });
     }
     for (unsigned long long ps = 0; ps < A.geo_passes; ++ps) {
-        res_sync<CL>();
+        res_sync<NC>();
         // columns: the row factors first, then the column factor of what they leave
         res_rows(MT, [&](int k, int o, int step, int n) {
             double lo = INFINITY, hi = 0.0;
@@ -161,10 +161,10 @@ __device__ __noinline__ void res_scale(ResShared &sh, const BatchArgs &A, double
             for (int j = 0, d = o; j < n; ++j, d += step)
                 if (MT.ci[d] != noneT) vT[d] = (vT[d] * fr[MT.ci[d]]) * f;
             fc[k] = f;
-            publish<CL>(fc + k);
+            publish<NC>(fc + k);
             cs[k] *= f;
         });
-        res_sync<CL>();
+        res_sync<NC>();
         const bool more = ps + 1 < A.geo_passes;
         res_rows(MA, [&](int k, int o, int step, int n) {
             const double f = fr[k];
@@ -180,14 +180,14 @@ __device__ __noinline__ void res_scale(ResShared &sh, const BatchArgs &A, double
             rs[k] *= f;
             if (more) {
                 fr[k] = factor_geo(lo, hi);
-                publish<CL>(fr + k);
+                publish<NC>(fr + k);
             }
         });
     }
     const unsigned long long steps = A.ruiz_iterations + (A.pc_enabled ? 1 : 0);
     for (unsigned long long it = 0; it < steps; ++it) {
         const bool pc = it == A.ruiz_iterations;  // Pock-Chambolle: sums in index order
-        auto factor = [&](const ResSide &M, const double *v, int none, int o, int step, int n, double alpha) {
+        auto factor = [&](const ResSide<uint16_t> &M, const double *v, int none, int o, int step, int n, double alpha) {
             if (!pc) {
                 double lo = INFINITY, hi = 0.0;
                 span(M.ci, v, none, o, step, n, lo, hi);
@@ -201,18 +201,18 @@ __device__ __noinline__ void res_scale(ResShared &sh, const BatchArgs &A, double
                 }
             return factor_of(s);
         };
-        res_sync<CL>();
+        res_sync<NC>();
         res_rows(MA, [&](int k, int o, int step, int n) { yn[k] = factor(MA, vA, noneA, o, step, n, A.pc_alpha); });
         res_rows(MT, [&](int k, int o, int step, int n) { xn[k] = factor(MT, vT, noneT, o, step, n, 2.0 - A.pc_alpha); });
         res_rows(MA, [&](int k, int, int, int) {
             fr[k] = yn[k];
-            publish<CL>(fr + k);
+            publish<NC>(fr + k);
         });
         res_rows(MT, [&](int k, int, int, int) {
             fc[k] = xn[k];
-            publish<CL>(fc + k);
+            publish<NC>(fc + k);
         });
-        res_sync<CL>();
+        res_sync<NC>();
         res_rows(MA, [&](int k, int o, int step, int n) {
             const double f = fr[k];
 #pragma unroll 4
@@ -228,7 +228,7 @@ __device__ __noinline__ void res_scale(ResShared &sh, const BatchArgs &A, double
             cs[k] *= f;
         });
     }
-    res_sync<CL>();
+    res_sync<NC>();
 }
 
 // The four norms (scaling.rs:186-201, solver.rs:317-318), each a sum in index order from -0.0:
@@ -288,7 +288,7 @@ struct ResTailStop {
 };
 
 struct ResBatchShared {
-    ResShared s;
+    ResShared<uint16_t> s;
     double bs, os;  // the scalar rescalings
     float next;     // the instance's number (below 2^24), by cluster_store
 };
@@ -301,14 +301,13 @@ __device__ __forceinline__ ResBatchPlaces res_batch_places(const ResBatchInst &I
 template <int NC, bool MIXED, bool ES>
 __device__ __noinline__ void res_batch_setup(const BatchArgs &A, const BatchRes &B, const ResBatchInst &I,
                                              unsigned char *scratch, ResBatchShared &bsh) {
-    constexpr bool CL = NC > 1;
-    ResShared &s = bsh.s;
+    ResShared<uint16_t> &s = bsh.s;
     const BatchInst &D = A.inst[I.id];
-    const int m = D.m, n = D.n, c = CL ? (int)cluster_rank() : 0;
+    const int m = D.m, n = D.n, c = res_rank<NC>();
     const ResBatchPlaces L = res_batch_places(I, m, n, MIXED, ES);
     const ResScratch W(I.sA[NC], I.sT[NC], m, n, D.nta, D.ntt, MIXED);
     auto src = [&](bool a) {
-        ResSrc q{};
+        ResSrc<uint16_t> q{};
         const int *most = a ? I.mostA : I.mostT;
         q.rows = a ? m : n;
         q.heavy = a ? I.heavyA : I.heavyT;
@@ -328,7 +327,7 @@ __device__ __noinline__ void res_batch_setup(const BatchArgs &A, const BatchRes 
         q.tiles = a ? A.a_tiles + D.ta : A.t_tiles + D.tt;
         return q;
     };
-    const ResSrc SA = src(true), ST = src(false);
+    const ResSrc<uint16_t> SA = src(true), ST = src(false);
     SolverPtrs g{};
     g.pk = (CheckQuad *)(scratch + W.pk);
     g.pky = (double2 *)(scratch + W.pky);
@@ -342,8 +341,8 @@ __device__ __noinline__ void res_batch_setup(const BatchArgs &A, const BatchRes 
     double *vecs = (double *)(scratch + W.vecs);
     const ResVecs vec{vecs, vecs + n, vecs + 2 * n, vecs + 3 * n, vecs + 3 * n + m};
     res_open(s, L, SA, ST, g, vec, (double *)(scratch + W.contrib), c);
-    const ResCtx &R = s.R;
-    const ResSide &MA = R.A, &MT = R.T;
+    const ResCtx<uint16_t> &R = s.R;
+    const ResSide<uint16_t> &MA = R.A, &MT = R.T;
     const SolverPtrs &S = R.S;
 
     // the entries as given, then the scaling passes on them
@@ -354,10 +353,10 @@ __device__ __noinline__ void res_batch_setup(const BatchArgs &A, const BatchRes 
     __syncthreads();
     // rs and cs over positions in pf and df, and in row order for the norms and the solution
     double *rs = vec.pf, *cs = vec.df, *grs = A.rs + D.mo, *gcs = A.cs + D.no;
-    res_scale<CL>(s, A, vA, vT, rs, cs);
+    res_scale<NC>(s, A, vA, vT, rs, cs);
     for (int k = MA.p0 + threadIdx.x; k < MA.p1; k += RES_BT) grs[MA.perm[k]] = rs[k];
     for (int k = MT.p0 + threadIdx.x; k < MT.p1; k += RES_BT) gcs[MT.perm[k]] = cs[k];
-    auto finish = [&](const ResSide &M, const double *v, double *gv, float *gv32) {
+    auto finish = [&](const ResSide<uint16_t> &M, const double *v, double *gv, float *gv32) {
         for (int i = threadIdx.x; i < M.slots; i += RES_BT) {
             const double x = v[i];
             if (ES) gv[i] = x;
@@ -366,7 +365,7 @@ __device__ __noinline__ void res_batch_setup(const BatchArgs &A, const BatchRes 
     };
     finish(MA, vA, gvA, MIXED ? SA.v32 + SA.s0[c] : nullptr);
     finish(MT, vT, gvT, MIXED ? ST.v32 + ST.s0[c] : nullptr);
-    res_sync<CL>();
+    res_sync<NC>();
     const double *oc = A.oc + D.no, *olv = A.olv + D.no, *ouv = A.ouv + D.no, *olc = A.olc + D.mo, *ouc = A.ouc + D.mo;
     double norms[4];
     res_norms(olc, ouc, oc, grs, gcs, m, n, norms);
@@ -417,9 +416,9 @@ __device__ __noinline__ void res_batch_setup(const BatchArgs &A, const BatchRes 
         vec.pf[k] = 1.0 / (f * bs);
         S.ya[k] = 0.0;
     }
-    res_sync<CL>();
+    res_sync<NC>();
     if (D.nnz > 0) res_power<NC, ES>(s, L, A.power_iterations, ppart);
-    res_sync<CL>();  // y is the power iteration's until here
+    res_sync<NC>();  // y is the power iteration's until here
     if (threadIdx.x == 0) {
         const bool numerical = D.nnz > 0 && s.st.error == ERR_NUMERICAL_POWER;
         const double norm_est = D.nnz > 0 ? sqrt(s.st.pi_lambda) * 1.01 : 1.0;
@@ -448,15 +447,15 @@ __device__ __noinline__ void res_batch_setup(const BatchArgs &A, const BatchRes 
         res_load_entries<float>(MA, MA.v32, L.valA, L.atA, L.xbar32);
         res_load_entries<float>(MT, MT.v32, L.valT, L.atT, L.y32);
     }
-    res_sync<CL>();
+    res_sync<NC>();
 }
 
 // The result and the solution in the original space (solver.rs:422-437).
-template <bool CL>
+template <int NC>
 __device__ __noinline__ void res_batch_finish(const BatchArgs &A, const ResBatchInst &I, ResBatchShared &bsh) {
-    const ResShared &s = bsh.s;
+    ResShared<uint16_t> &s = bsh.s;
     const BatchInst &D = A.inst[I.id];
-    const ResSide &MA = s.R.A, &MT = s.R.T;
+    const ResSide<uint16_t> &MA = s.R.A, &MT = s.R.T;
     const double bs = bsh.bs, os = bsh.os, *grs = A.rs + D.mo, *gcs = A.cs + D.no;
     double *ox = A.ox + D.no, *oy = A.oy + D.mo;
     for (int k = MT.p0 + threadIdx.x; k < MT.p1; k += RES_BT) {
@@ -467,7 +466,7 @@ __device__ __noinline__ void res_batch_finish(const BatchArgs &A, const ResBatch
         const int i = MA.perm[k];
         oy[i] = s.R.S.yt[k] * grs[i] / os;
     }
-    if (threadIdx.x == 0 && (!CL || cluster_rank() == 0)) {
+    if (threadIdx.x == 0 && res_rank<NC>() == 0) {
         const DevState &st = s.st;
         sp_batch_result r;
         const double sign = D.maximize ? -1.0 : 1.0;
@@ -483,7 +482,7 @@ __device__ __noinline__ void res_batch_finish(const BatchArgs &A, const ResBatch
         r.handed_off = st.handoff ? 2 : 0;  // 2: the host finishes it
         A.res[I.id] = r;
     }
-    res_sync<CL>();
+    res_sync<NC>();
 }
 
 // One class of instances: clusters of NC CTAs take them from the class's counter.
@@ -491,18 +490,17 @@ template <int NC, bool MIXED>
 __global__ void __launch_bounds__(RES_BT, 1)
     k_batch_res(const __grid_constant__ BatchArgs A, const __grid_constant__ BatchRes B,
                 const __grid_constant__ ResBatchClass K) {
-    constexpr bool CL = NC > 1;
     __shared__ ResBatchShared b;
     unsigned char *scratch = K.scratch + (size_t)(blockIdx.x / NC) * K.scratch_bytes;
     const ResTailStop stop{&A};
     for (;;) {
-        if (threadIdx.x == 0 && (!CL || cluster_rank() == 0)) {
+        if (threadIdx.x == 0 && res_rank<NC>() == 0) {
             b.next = (float)batch_claim(A, K.counter, K.count);
-            publish<CL>(&b.next);
+            publish<NC>(&b.next);
         }
-        res_sync<CL>();
+        res_sync<NC>();
         const int slot = (int)b.next;
-        res_sync<CL>();
+        res_sync<NC>();
         if (slot >= K.count) return;
         const ResBatchInst &I = K.inst[slot];
         auto solve = [&](auto in_shared) {
@@ -511,7 +509,7 @@ __global__ void __launch_bounds__(RES_BT, 1)
             const ResBatchPlaces L = res_batch_places(I, b.s.R.A.rows, b.s.R.T.rows, MIXED, ES);
             if constexpr (MIXED) {
                 res_epochs<NC, true, ES>(b.s, L, stop);
-                res_sync<CL>();
+                res_sync<NC>();
                 if (ES && !b.s.st.done) {
                     res_load_entries<double>(b.s.R.A, b.s.R.A.v, L.valA, L.atA, L.xbar);
                     res_load_entries<double>(b.s.R.T, b.s.R.T.v, L.valT, L.atT, L.y);
@@ -519,11 +517,11 @@ __global__ void __launch_bounds__(RES_BT, 1)
                 }
             }
             res_epochs<NC, false, ES>(b.s, L, stop);
-            res_sync<CL>();
+            res_sync<NC>();
         };
         if (I.es) solve(std::true_type{});
         else solve(std::false_type{});
-        res_batch_finish<CL>(A, I, b);
+        res_batch_finish<NC>(A, I, b);
     }
 }
 

@@ -18,6 +18,7 @@ struct sp_ctx {
     double *d_partials = nullptr;  // stage-one partials of the trait-method reductions
     double *d_result = nullptr;    // their final values
     double *h_result = nullptr;    // pinned copy read by the host
+    bool shared = false;           // one of several contexts that solve at the same time (a server's)
     int *d_tiles = nullptr;        // work counters of the tile launches on `stream` (tiles.cuh: run_tiles)
 };
 

@@ -53,14 +53,14 @@ constexpr int RES_MAX_ROWS = 65534;     // 16-bit positions, and one for the pad
 static_assert(RES_BT % NT == 0 && RES_GROUPS >= 1, "whole tile groups");
 
 // A task: x = its first slot and y = its first position (both from its CTA's first), z = its
-// rows, w = the width of a slice (even), or minus the chunks of each of a group of warp rows.
+// rows, w = the width of a slice, or minus the chunks of each of a group of warp rows (both
+// even in a plan of pairs).
 using ResTask = int4;
 
-// The plan of one matrix (host).
-struct ResPlan {
-    std::vector<uint16_t> perm;   // [rows] the row at each position
-    std::vector<uint16_t> inv;    // [rows] the position of each row
+// The plan of one matrix (host), but for which row is at which position.
+struct ResCuts {
     std::vector<ResTask> tasks;   // by CTA, then warp
+    std::vector<int> first;       // [tasks] each task's first row in the order of decreasing length
     std::vector<int> wt;          // [ctas * RES_W + 1] first task of each warp
     std::vector<int> p0, s0;      // [ctas + 1] first position and first slot of each CTA
     int64_t slots = 0;
@@ -68,53 +68,68 @@ struct ResPlan {
     bool heavy = false;
 };
 
-// Host: the plan of the matrix with row pointers rp, for a cluster of `ctas` CTAs.
-template <class I>
-inline void res_plan(const I *rp, int rows, int ctas, ResPlan *P) {
-    // rows by decreasing length, ties in row order (a counting sort)
-    int64_t maxlen = 0;
-    for (int r = 0; r < rows; ++r) maxlen = std::max<int64_t>(maxlen, (int64_t)(rp[r + 1] - rp[r]));
-    std::vector<int> start((size_t)maxlen + 2, 0), order((size_t)rows);
-    for (int r = 0; r < rows; ++r) ++start[(size_t)(maxlen - (int64_t)(rp[r + 1] - rp[r])) + 1];
-    for (size_t l = 1; l < start.size(); ++l) start[l] += start[l - 1];
-    for (int r = 0; r < rows; ++r) order[(size_t)start[(size_t)(maxlen - (int64_t)(rp[r + 1] - rp[r]))]++] = r;
+// Host: cuts the rows, `count[l]` of them with l entries, into tasks and deals these to the
+// warps of `ctas` CTAs. pairs: widths and chunks are even. Nothing else about the rows matters.
+inline void res_cut(const std::vector<int> &count, int ctas, bool pairs, ResCuts *P) {
+    const int odd = pairs ? 1 : 0;
     struct Cut {
         int first, cnt, width, slots, cost;
     };
     std::vector<Cut> cuts;
-    auto len_of = [&](int o) { return (int)(rp[order[o] + 1] - rp[order[o]]); };
     int o = 0;
-    while (o < rows && len_of(o) > SEQ_MAX) {  // rows of the same number of chunks
-        const int ch = (len_of(o) + 63) / 64 * 2, first = o;  // an even number
-        while (o < rows && o - first < std::max(1, RES_HEAVY_CHUNKS / ch) && len_of(o) > SEQ_MAX &&
-               (len_of(o) + 63) / 64 * 2 == ch)
-            ++o;
-        const int cnt = o - first;
-        cuts.push_back(Cut{first, cnt, -ch, 32 * ch * cnt, 8 + cnt * (4 + ch)});
+    int l = (int)count.size() - 1;
+    auto chunks = [&](int len) { return ((len + 31) / 32 + odd) & ~odd; };
+    while (l > SEQ_MAX) {  // groups of rows of the same number of chunks
+        const int ch = chunks(l), most = std::max(1, RES_HEAVY_CHUNKS / ch);
+        int n = 0;
+        for (; l > SEQ_MAX && chunks(l) == ch; --l) n += count[l];
+        for (; n > 0; n -= std::min(n, most)) {
+            const int cnt = std::min(n, most);
+            cuts.push_back(Cut{o, cnt, -ch, 32 * ch * cnt, 8 + cnt * (4 + ch)});
+            o += cnt;
+        }
     }
-    while (o < rows) {
-        const int cnt = std::min(32, rows - o), w = (len_of(o) + 1) & ~1;
-        cuts.push_back(Cut{o, cnt, w, 32 * w, 8 + w});
-        o += cnt;
+    int rest = 0;  // rows that the open slice still takes
+    for (; l >= 0; --l)
+        for (int n = count[l]; n > 0;) {
+            if (rest == 0) {
+                const int w = (l + odd) & ~odd;
+                cuts.push_back(Cut{o, 0, w, 32 * w, 8 + w});
+                rest = 32;
+            }
+            const int k = std::min(n, rest);
+            cuts.back().cnt += k;
+            o += k;
+            rest -= k;
+            n -= k;
+        }
+    // a few tasks to a warp: longest first, each to the least loaded warp (ties: CTA after CTA);
+    // many: in turn, there and back. Turn k counts CTAs fastest: warp k / ctas of CTA k % ctas.
+    const int nw = ctas * RES_W, nc = (int)cuts.size();
+    std::vector<int> of((size_t)nc), by((size_t)nc);
+    for (int c = 0; c < nc; ++c) by[c] = c;
+    if (nc <= 16 * nw) {
+        std::stable_sort(by.begin(), by.end(), [&](int a, int b) { return cuts[a].cost > cuts[b].cost; });
+        using Load = std::pair<int, int>;
+        std::priority_queue<Load, std::vector<Load>, std::greater<Load>> heap;
+        for (int k = 0; k < nw; ++k) heap.push({0, k});
+        for (int c : by) {
+            const Load x = heap.top();
+            heap.pop();
+            of[c] = x.second;
+            heap.push({x.first + cuts[c].cost, x.second});
+        }
+    } else {
+        for (int c = 0; c < nc; ++c) of[c] = (c / nw) & 1 ? nw - 1 - c % nw : c % nw;
     }
-    std::stable_sort(cuts.begin(), cuts.end(), [](const Cut &a, const Cut &b) { return a.cost > b.cost; });
-    // longest first, each to the least loaded warp (ties: CTA after CTA)
-    const int nw = ctas * RES_W;
-    using Load = std::pair<int, int>;
-    std::priority_queue<Load, std::vector<Load>, std::greater<Load>> heap;
-    for (int k = 0; k < nw; ++k) heap.push({0, k});
-    std::vector<std::vector<int>> mine((size_t)nw);
-    for (int c = 0; c < (int)cuts.size(); ++c) {
-        const Load l = heap.top();
-        heap.pop();
-        const int k = l.second;  // k counts CTAs fastest: warp k / ctas of CTA k % ctas
-        mine[(size_t)(k % ctas) * RES_W + k / ctas].push_back(c);
-        heap.push({l.first + cuts[c].cost, k});
-    }
-    P->perm.resize((size_t)rows);
-    P->inv.resize((size_t)rows);
-    P->tasks.clear();
     P->wt.assign((size_t)nw + 1, 0);
+    auto warp_of = [&](int c) { return of[c] % ctas * RES_W + of[c] / ctas; };
+    for (int c = 0; c < nc; ++c) ++P->wt[warp_of(c) + 1];
+    for (int w = 0; w < nw; ++w) P->wt[w + 1] += P->wt[w];
+    std::vector<int> at(P->wt.begin(), P->wt.end() - 1), list((size_t)nc);
+    for (int c : by) list[at[warp_of(c)]++] = c;
+    P->tasks.resize((size_t)nc);
+    P->first.resize((size_t)nc);
     P->p0.assign((size_t)ctas + 1, 0);
     P->s0.assign((size_t)ctas + 1, 0);
     int pos = 0, slot = 0;
@@ -124,19 +139,15 @@ inline void res_plan(const I *rp, int rows, int ctas, ResPlan *P) {
             P->p0[c] = pos;
             P->s0[c] = slot;
         }
-        P->wt[w] = (int)P->tasks.size();
-        for (int k : mine[w]) {
-            const Cut &q = cuts[k];
+        for (int t = P->wt[w]; t < P->wt[w + 1]; ++t) {
+            const Cut &q = cuts[list[t]];
             P->heavy |= q.width < 0;
-            P->tasks.push_back(make_int4(slot - P->s0[c], pos - P->p0[c], q.cnt, q.width));
-            for (int i = 0; i < q.cnt; ++i, ++pos) {
-                P->perm[pos] = (uint16_t)order[q.first + i];
-                P->inv[order[q.first + i]] = (uint16_t)pos;
-            }
+            P->tasks[t] = make_int4(slot - P->s0[c], pos - P->p0[c], q.cnt, q.width);
+            P->first[t] = q.first;
+            pos += q.cnt;
             slot += q.slots;
         }
     }
-    P->wt[nw] = (int)P->tasks.size();
     P->p0[ctas] = pos;
     P->s0[ctas] = slot;
     P->slots = slot;
@@ -145,6 +156,34 @@ inline void res_plan(const I *rp, int rows, int ctas, ResPlan *P) {
         P->most_slots = std::max(P->most_slots, P->s0[c + 1] - P->s0[c]);
         P->most_tasks = std::max(P->most_tasks, P->wt[(c + 1) * RES_W] - P->wt[c * RES_W]);
     }
+}
+
+// The whole plan of a small matrix.
+struct ResPlan : ResCuts {
+    std::vector<uint16_t> perm;   // [rows] the row at each position
+    std::vector<uint16_t> inv;    // [rows] the position of each row
+};
+
+// Host: the plan of the matrix with row pointers rp, for `ctas` CTAs.
+template <class I>
+inline void res_plan(const I *rp, int rows, int ctas, bool pairs, ResPlan *P) {
+    int maxlen = 0;
+    for (int r = 0; r < rows; ++r) maxlen = std::max(maxlen, (int)(rp[r + 1] - rp[r]));
+    std::vector<int> count((size_t)maxlen + 1, 0), start((size_t)maxlen + 2, 0), order((size_t)rows);
+    for (int r = 0; r < rows; ++r) ++count[(size_t)(rp[r + 1] - rp[r])];
+    res_cut(count, ctas, pairs, P);
+    // rows by decreasing length, ties in row order
+    for (int l = maxlen; l >= 0; --l) start[(size_t)(maxlen - l) + 1] = start[(size_t)(maxlen - l)] + count[l];
+    for (int r = 0; r < rows; ++r) order[(size_t)start[(size_t)(maxlen - (int)(rp[r + 1] - rp[r]))]++] = r;
+    P->perm.resize((size_t)rows);
+    P->inv.resize((size_t)rows);
+    for (int c = 0; c < ctas; ++c)
+        for (int t = P->wt[c * RES_W]; t < P->wt[(c + 1) * RES_W]; ++t)
+            for (int i = 0; i < P->tasks[t].z; ++i) {
+                const int pos = P->p0[c] + P->tasks[t].y + i, r = order[P->first[t] + i];
+                P->perm[pos] = (uint16_t)r;
+                P->inv[r] = (uint16_t)pos;
+            }
 }
 
 // ------------------------------------------------------------------ cluster primitives
@@ -159,16 +198,25 @@ __device__ __forceinline__ unsigned cluster_size() {
     asm volatile("mov.u32 %0, %%cluster_nctarank;" : "=r"(r));
     return r;
 }
-// The barrier of the whole cluster (CL) or of the CTA: what was written before it, in shared
-// memory of any CTA and in global memory, is visible after it.
-template <bool CL>
+// The barrier of a solve's CTAs, a cluster of NC or one: what was written before it, in shared
+// memory of any of them and in global memory, is visible after it.
+template <int NC>
 __device__ __forceinline__ void res_sync() {
-    if constexpr (CL) {
+    if constexpr (NC > 1) {
         asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
         asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
     } else {
         __syncthreads();
     }
+}
+// This CTA's number among the solve's, and how many there are (NC = 0: the grid).
+template <int NC>
+__device__ __forceinline__ int res_rank() {
+    return NC > 1 ? (int)cluster_rank() : NC == 1 ? 0 : (int)blockIdx.x;
+}
+template <int NC>
+__device__ __forceinline__ int res_size() {
+    return NC > 0 ? NC : (int)gridDim.x;
 }
 // Writes v to the place of shared variable *p in CTA `rank` of the cluster.
 __device__ __forceinline__ void cluster_store(double *p, unsigned rank, double v) {
@@ -182,9 +230,9 @@ __device__ __forceinline__ void cluster_store(float *p, unsigned rank, float v) 
     asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(a), "f"(v) : "memory");
 }
 // Copies this thread's own *p to the same place in the other CTAs of the cluster.
-template <bool CL, class T>
+template <int NC, class T>
 __device__ __forceinline__ void publish(T *p) {
-    if constexpr (CL) {
+    if constexpr (NC > 1) {
         const unsigned me = cluster_rank(), n = cluster_size();
         const T v = *p;
         for (unsigned r = 1; r < n; ++r) cluster_store(p, me + r < n ? me + r : me + r - n, v);
@@ -231,36 +279,39 @@ struct ResPlaces {
 
 // One matrix as a CTA sees it: its part of the plan, its entries in global memory (positions
 // and values; in shared memory too where the kernel says so), and what the fold needs.
+template <class IX>
 struct ResSide {
     int rows, p0, p1;       // all rows; this CTA's positions
     int slots, ntasks;      // this CTA's
     int heavy;              // whether the matrix has warp rows
     int ntiles;
     int tasks, wt;          // their places in dynamic shared memory
-    const uint16_t *ci;     // [slots]
+    const IX *ci;           // [slots]
     const double *v;
     const float *v32;
-    const uint16_t *perm;   // all positions
+    const IX *perm;         // all positions
     const int *rp;          // the CSR row pointers, for the fold's row lengths
     const Tile *tiles;
 };
 
 // One matrix in global memory: the whole plan and all slots.
+template <class IX>
 struct ResSrc {
     int rows, heavy, ntiles;
     int most_rows, most_slots, most_tasks;
     const ResTask *tasks;
     const int *wt, *p0, *s0;
-    const uint16_t *perm;
-    uint16_t *ci;
+    const IX *perm;
+    IX *ci;
     double *v;
     float *v32;
     const int *rp;
     const Tile *tiles;
 };
 
+template <class IX>
 struct ResCtx {
-    ResSide A, T;           // A' (rows i) and A'ᵀ (rows j)
+    ResSide<IX> A, T;       // A' (rows i) and A'ᵀ (rows j)
     SolverPtrs S;           // vectors over positions (in any memory)
     double *contrib;        // [8 rows] row contributions of a pass, in row order
     double *contribD, *contribT;
@@ -274,8 +325,9 @@ struct ResVecs {
 
 // A CTA's shared variables: the problem's arrays, its copy of the solver's state, and what the
 // epochs need between their iterations (kept out of the iterations' registers).
+template <class IX>
 struct ResShared {
-    ResCtx R;
+    ResCtx<IX> R;
     DevState st;
     DevParams prm;
     unsigned long long until;   // iterations at which to stop
@@ -294,8 +346,9 @@ __device__ __forceinline__ T &dsm_at(int place) {
     return *reinterpret_cast<T *>(dsm + place);
 }
 
-__device__ __forceinline__ ResSide res_side(const ResSrc &M, int c, int tasks, int wt) {
-    ResSide d;
+template <class IX>
+__device__ __forceinline__ ResSide<IX> res_side(const ResSrc<IX> &M, int c, int tasks, int wt) {
+    ResSide<IX> d;
     d.rows = M.rows;
     d.p0 = M.p0[c];
     d.p1 = M.p0[c + 1];
@@ -316,11 +369,11 @@ __device__ __forceinline__ ResSide res_side(const ResSrc &M, int c, int tasks, i
 
 // Sets sh.R up for CTA c and copies the plan into shared memory (not the entries). R.S keeps
 // its other pointers. Ends with a barrier.
-template <int PT, int PA>
-__device__ inline void res_open(ResShared &sh, const ResPlaces<PT, PA> &L, const ResSrc &A, const ResSrc &T,
+template <int PT, int PA, class IX>
+__device__ inline void res_open(ResShared<IX> &sh, const ResPlaces<PT, PA> &L, const ResSrc<IX> &A, const ResSrc<IX> &T,
                                 const SolverPtrs &g, const ResVecs &vec, double *contrib, int c) {
     if (threadIdx.x == 0) {
-        ResCtx &R = sh.R;
+        ResCtx<IX> &R = sh.R;
         R.A = res_side(A, c, L.tasksA, L.wtA);
         R.T = res_side(T, c, L.tasksT, L.wtT);
         R.S = g;
@@ -357,7 +410,7 @@ __device__ inline void res_open(ResShared &sh, const ResPlaces<PT, PA> &L, const
         S.pk[T.rows] = CheckQuad{1.0, 1.0, 1.0, 1.0};
         S.pky[A.rows] = make_double2(1.0, 1.0);
     }
-    for (const ResSrc *M : {&A, &T}) {
+    for (const ResSrc<IX> *M : {&A, &T}) {
         const int *wt = M->wt + c * RES_W;
         const int tasks = M == &A ? L.tasksA : L.tasksT, to = M == &A ? L.wtA : L.wtT, n = wt[RES_W] - wt[0];
         for (int i = threadIdx.x; i < n; i += RES_BT) (&dsm_at<ResTask>(tasks))[i] = M->tasks[wt[0] + i];
@@ -368,8 +421,8 @@ __device__ inline void res_open(ResShared &sh, const ResPlaces<PT, PA> &L, const
 
 // The CTA's entries of one matrix into shared memory; `base` is the place of the vector they
 // gather.
-template <class VT>
-__device__ inline void res_load_entries(const ResSide &M, const VT *v, int val, int at, int base) {
+template <class VT, class IX>
+__device__ inline void res_load_entries(const ResSide<IX> &M, const VT *v, int val, int at, int base) {
     for (int i = threadIdx.x; i < M.slots; i += RES_BT) (&dsm_at<VT>(val))[i] = v[i];
     for (int i = threadIdx.x; i < M.slots / 2; i += RES_BT) {
         const int o = (i & ~31) * 2 + (i & 31);
@@ -397,7 +450,7 @@ struct ResEntries {
     int val, at;         // ES: their places; else at = the place of the gathered vector
     const uint16_t *ci;
     const VT *v;
-    __device__ __forceinline__ ResEntries(const ResSide &M, const VT *vals, int val_, int at_, int base) {
+    __device__ __forceinline__ ResEntries(const ResSide<uint16_t> &M, const VT *vals, int val_, int at_, int base) {
         const int lane = threadIdx.x & 31;
         const unsigned b = (unsigned)base / (unsigned)sizeof(VT);
         if constexpr (ES) {
@@ -575,13 +628,13 @@ __device__ __forceinline__ void res_tree(double (&v)[NP], double *sh) {
 
 // The tile partials [ntiles][NP] of a pass from its contributions, in the tile engine's
 // order: thread u of a tile its short rows u, u + NT, ..., lane 0 of warp w the warp rows
-// w, w + 8, ..., then the block tree. Groups of NT threads take a tile each, over the whole
-// cluster. Contributions are read from L2 (another CTA may have written them).
-template <bool CL, int NP>
-__device__ __forceinline__ void res_fold(const ResSide &M, const double *contrib, double *part, double *sh) {
+// w, w + 8, ..., then the block tree. Groups of NT threads take a tile each, over all of the
+// solve's CTAs. Contributions are read from L2 (another CTA may have written them).
+template <int NC, int NP, class IX>
+__device__ __forceinline__ void res_fold(const ResSide<IX> &M, const double *contrib, double *part, double *sh) {
     constexpr int W = NT / 32;
     const int g = threadIdx.x / NT, tid = threadIdx.x % NT, warp = tid >> 5, lane = tid & 31;
-    const int c = CL ? (int)cluster_rank() : 0, nc = CL ? (int)cluster_size() : 1;
+    const int c = res_rank<NC>(), nc = res_size<NC>();
     const int step = nc * RES_GROUPS;
     double *gsh = sh + g * NP * W;
     for (int base = c * RES_GROUPS; base < M.ntiles; base += step) {
@@ -631,7 +684,7 @@ __device__ __forceinline__ void res_total(const double *part, int tiles, double 
 // ------------------------------------------------------------------ the checks' passes
 
 // The solver's passes on positions. Their row() is the solver's.
-template <bool CL, bool LO, int MODE>
+template <int NC, bool LO, int MODE>
 struct ResPrimal : PrimalPass<LO, MODE> {
     using Base = PrimalPass<LO, MODE>;
     using Pre = typename Base::Pre;
@@ -648,7 +701,7 @@ struct ResPrimal : PrimalPass<LO, MODE> {
     __device__ __forceinline__ void publish_at(int) const {}  // the dual pass gathers the column records
 };
 
-template <bool CL, bool LO, int MODE>
+template <int NC, bool LO, int MODE>
 struct ResDual : DualPass<LO, MODE> {
     using Base = DualPass<LO, MODE>;
     using Pre = typename Base::Pre;
@@ -672,8 +725,8 @@ struct ResDual : DualPass<LO, MODE> {
     }
     __device__ __forceinline__ void publish_at(int k) const {
         if constexpr (MODE == 1) {
-            if constexpr (LO) publish<CL>(this->s.y32 + k);
-            else publish<CL>(this->s.y + k);
+            if constexpr (LO) publish<NC>(this->s.y32 + k);
+            else publish<NC>(this->s.y + k);
         }
     }
 };
@@ -692,8 +745,8 @@ struct ResCheckT : CheckPassT {
 
 // A check pass over this CTA's rows of M, its entries from global memory: each row's NP
 // contributions are left in contrib ([NP][rows], row order).
-template <class Op>
-__device__ __forceinline__ void res_pass(const ResSide &M, const Op &op, double *contrib) {
+template <class Op, class IX>
+__device__ __forceinline__ void res_pass(const ResSide<IX> &M, const Op &op, double *contrib) {
     using VT = typename Op::VT;
     using ST = typename Op::ST;
     constexpr int G = Op::G, NP = Op::NP;
@@ -711,18 +764,21 @@ __device__ __forceinline__ void res_pass(const ResSide &M, const Op &op, double 
         if (live) pre = op.pre_at(k);
         double s[G];
         int o = t.x + lane;
-        auto add2 = [&](SlotSums<G, Op::F32> &acc) {
-            ST p[2][G];
+        auto add = [&](SlotSums<G, Op::F32> &acc, auto count) {
+            constexpr int N = decltype(count)::value;
+            ST p[N][G];
 #pragma unroll
-            for (int u = 0; u < 2; ++u) op.prod(M.ci[o + 32 * u], vals[o + 32 * u], p[u]);
+            for (int u = 0; u < N; ++u) op.prod(M.ci[o + 32 * u], vals[o + 32 * u], p[u]);
 #pragma unroll
-            for (int u = 0; u < 2; ++u) acc.add(p[u]);
+            for (int u = 0; u < N; ++u) acc.add(p[u]);
         };
         SlotSums<G, Op::F32> acc;
         if (t.w >= 0) {
             acc.clear();
+            int j = 0;
 #pragma unroll 2
-            for (int j = 0; j < t.w; j += 2, o += 64) add2(acc);
+            for (; j + 2 <= t.w; j += 2, o += 64) add(acc, std::integral_constant<int, 2>{});
+            if (j < t.w) add(acc, std::integral_constant<int, 1>{});
 #pragma unroll
             for (int q = 0; q < G; ++q) s[q] = acc.get(q);
         } else {
@@ -759,16 +815,16 @@ __device__ __forceinline__ void res_pass(const ResSide &M, const Op &op, double 
     }
 }
 
-template <bool CL, bool LO, int MODE>
-__device__ __forceinline__ void res_primal(const ResCtx &R, const IterScalars &sc) {
-    ResPrimal<CL, LO, MODE> o{};
+template <int NC, bool LO, int MODE, class IX>
+__device__ __forceinline__ void res_primal(const ResCtx<IX> &R, const IterScalars &sc) {
+    ResPrimal<NC, LO, MODE> o{};
     o.s = R.S;
     o.sc = sc;
     res_pass(R.T, o, R.contrib);
 }
-template <bool CL, bool LO, int MODE>
-__device__ __forceinline__ void res_dual(const ResCtx &R, const IterScalars &sc) {
-    ResDual<CL, LO, MODE> o{};
+template <int NC, bool LO, int MODE, class IX>
+__device__ __forceinline__ void res_dual(const ResCtx<IX> &R, const IterScalars &sc) {
+    ResDual<NC, LO, MODE> o{};
     o.s = R.S;
     o.sc = sc;
     res_pass(R.A, o, R.contribD);
@@ -832,7 +888,7 @@ struct ResPeers {
 
 // `its` FUSED iterations from Halpern counter k0.
 template <int NC, bool LO, bool ES, int PT, int PA>
-__device__ __forceinline__ void res_iterate(ResShared &sh, const ResPlaces<PT, PA> &L, unsigned long long k0,
+__device__ __forceinline__ void res_iterate(ResShared<uint16_t> &sh, const ResPlaces<PT, PA> &L, unsigned long long k0,
                                             unsigned long long its) {
     using VT = typename std::conditional<LO, float, double>::type;
     using P = ResPlaces<PT, PA>;
@@ -902,16 +958,17 @@ __device__ __forceinline__ void res_iterate(ResShared &sh, const ResPlaces<PT, P
             if (t0 < t1) primal((&dsm_at<ResTask>(L.tasksT))[t0], &hT);
 #pragma unroll 1
             for (int ti = t0 + 1; ti < t1; ++ti) primal((&dsm_at<ResTask>(L.tasksT))[ti], nullptr);
-            res_sync<(NC > 1)>();
+            res_sync<NC>();
             if (a0 < a1) dual((&dsm_at<ResTask>(L.tasksA))[a0], &hA);
 #pragma unroll 1
             for (int ti = a0 + 1; ti < a1; ++ti) dual((&dsm_at<ResTask>(L.tasksA))[ti], nullptr);
-            res_sync<(NC > 1)>();
+            res_sync<NC>();
         }
     }
 }
 
-__device__ __forceinline__ IterScalars res_scalars(const ResShared &sh, double w) {
+template <class IX>
+__device__ __forceinline__ IterScalars res_scalars(const ResShared<IX> &sh, double w) {
     IterScalars sc;
     sc.tau = sh.prm.eta / sh.st.omega;
     sc.sigma = sh.prm.eta * sh.st.omega;
@@ -922,19 +979,19 @@ __device__ __forceinline__ IterScalars res_scalars(const ResShared &sh, double w
 
 // The k = 0 iteration that opens an epoch: both passes with their residual sums, x's
 // Halpern step, and the anchor's residual (solver.rs:341-346). Non-finite iterates end the solve.
-template <bool CL, bool LO>
-__device__ __noinline__ void res_first(ResShared &sh) {
-    const ResCtx &R = sh.R;
+template <int NC, bool LO, class IX>
+__device__ __noinline__ void res_first(ResShared<IX> &sh) {
+    const ResCtx<IX> &R = sh.R;
     const IterScalars sc = res_scalars(sh, 1.0 / 2.0);
-    res_primal<CL, LO, 1>(R, sc);
-    res_sync<CL>();
-    res_dual<CL, LO, 1>(R, sc);
+    res_primal<NC, LO, 1>(R, sc);
+    res_sync<NC>();
+    res_dual<NC, LO, 1>(R, sc);
     for (int k = R.T.p0 + threadIdx.x; k < R.T.p1; k += RES_BT)
         R.S.x[k] = halpern(R.S.x[k], R.S.xt[k], R.S.xa[k], sc.w, sc.rho);
-    res_sync<CL>();
-    res_fold<CL, NP_P0>(R.T, R.contrib, R.S.partP0, sh.sh);
-    res_fold<CL, NP_D0>(R.A, R.contribD, R.S.partD0, sh.sh);
-    res_sync<CL>();
+    res_sync<NC>();
+    res_fold<NC, NP_P0>(R.T, R.contrib, R.S.partP0, sh.sh);
+    res_fold<NC, NP_D0>(R.A, R.contribD, R.S.partD0, sh.sh);
+    res_sync<NC>();
     double P0[NP_P0], D0[NP_D0];
     res_total<NP_P0>(R.S.partP0, R.T.ntiles, P0, sh.sh);
     res_total<NP_D0>(R.S.partD0, R.A.ntiles, D0, sh.sh);
@@ -957,32 +1014,32 @@ __device__ __noinline__ void res_first(ResShared &sh) {
 // The check iteration that ends an epoch of E iterations: its passes, the decisions (every CTA
 // takes the same ones from the same sums, on its own copy of the state), and the Halpern step
 // or the restart's copies. `stop` says whether an unfinished solve stops here for the batch's
-// hand-off: one CTA asks it, so that all of them agree.
-template <bool CL, bool LO, class Stop>
-__device__ __noinline__ void res_check(ResShared &sh, unsigned long long E, Stop stop) {
-    const ResCtx &R = sh.R;
+// hand-off: one CTA of a cluster asks it, so that all of them agree.
+template <int NC, bool LO, class IX, class Stop>
+__device__ __noinline__ void res_check(ResShared<IX> &sh, unsigned long long E, Stop stop) {
+    const ResCtx<IX> &R = sh.R;
     const SolverPtrs &S = R.S;
     DevState *st = &sh.st;
-    if (threadIdx.x == 0 && (!CL || cluster_rank() == 0)) {
+    if (threadIdx.x == 0 && (NC == 1 || cluster_rank() == 0)) {
         sh.stop = stop() ? 1.0f : 0.0f;
-        publish<CL>(&sh.stop);
+        publish<NC>(&sh.stop);
     }
     {
         const IterScalars sc = res_scalars(sh, 0.0);
-        res_primal<CL, LO, 2>(R, sc);
-        res_sync<CL>();
-        res_dual<CL, LO, 2>(R, sc);
-        res_sync<CL>();
+        res_primal<NC, LO, 2>(R, sc);
+        res_sync<NC>();
+        res_dual<NC, LO, 2>(R, sc);
+        res_sync<NC>();
         ResCheckT o{};
         o.s = S;
         o.inv_tau = 1.0 / sc.tau;
         res_pass(R.T, o, R.contribT);
     }
-    res_fold<CL, NP_P>(R.T, R.contrib, S.partP, sh.sh);
-    res_fold<CL, NP_D>(R.A, R.contribD, S.partD, sh.sh);
-    res_sync<CL>();
-    res_fold<CL, NP_T>(R.T, R.contribT, S.partT, sh.sh);
-    res_sync<CL>();
+    res_fold<NC, NP_P>(R.T, R.contrib, S.partP, sh.sh);
+    res_fold<NC, NP_D>(R.A, R.contribD, S.partD, sh.sh);
+    res_sync<NC>();
+    res_fold<NC, NP_T>(R.T, R.contribT, S.partT, sh.sh);
+    res_sync<NC>();
     double P[NP_P], D[NP_D], T[NP_T];
     res_total<NP_P>(S.partP, R.T.ntiles, P, sh.sh);
     res_total<NP_D>(S.partD, R.A.ntiles, D, sh.sh);
@@ -992,7 +1049,7 @@ __device__ __noinline__ void res_check(ResShared &sh, unsigned long long E, Stop
         sp_check_record rec;
         check_decide(st, &sh.prm, P, D, T, st->k + E - 1, st->total + E, &bad, &rec);
         if (!bad && sh.trace) {
-            if (!CL || cluster_rank() == 0)
+            if (res_rank<NC>() == 0)
                 if ((long long)st->checks - 1 < sh.trace_cap) sh.trace[st->checks - 1] = rec;
             st->trace_len = st->checks;
         }
@@ -1016,31 +1073,30 @@ __device__ __noinline__ void res_check(ResShared &sh, unsigned long long E, Stop
         if (rs) v = S.ya[k] = S.yt[k];
         else v = halpern(S.y[k], S.yt[k], S.ya[k], w, rho);
         S.y[k] = v;
-        publish<CL>(S.y + k);
+        publish<NC>(S.y + k);
         if (y32) {
             S.y32[k] = (float)v;
-            publish<CL>(S.y32 + k);
+            publish<NC>(S.y32 + k);
         }
     }
-    res_sync<CL>();
+    res_sync<NC>();
 }
 
 // Epochs of check_every iterations (the last one cut at max_iterations), each ended by its
 // check, until the state is done, its total has reached sh.until, or (mixed form) the other
 // precision is due: LO runs the FP32 phase.
 template <int NC, bool LO, bool ES, int PT, int PA, class Stop>
-__device__ __forceinline__ void res_epochs(ResShared &sh, const ResPlaces<PT, PA> &L, Stop stop) {
-    constexpr bool CL = NC > 1;
+__device__ __forceinline__ void res_epochs(ResShared<uint16_t> &sh, const ResPlaces<PT, PA> &L, Stop stop) {
     while (!sh.st.done && sh.st.total < sh.until && LO == (sh.mixed && !sh.st.fp64)) {
         unsigned long long E = sh.prm.max_iterations > sh.st.total ? sh.prm.max_iterations - sh.st.total : 1;
         if (sh.prm.check_every && sh.prm.check_every < E) E = sh.prm.check_every;
         const bool first = sh.st.k == 0 && E > 1;
         if (first) {
-            res_first<CL, LO>(sh);
+            res_first<NC, LO>(sh);
             if (sh.st.done) break;
         }
         res_iterate<NC, LO, ES>(sh, L, sh.st.k + first, E - 1 - first);
-        res_check<CL, LO>(sh, E, stop);
+        res_check<NC, LO>(sh, E, stop);
     }
 }
 
@@ -1050,10 +1106,9 @@ __device__ __forceinline__ void res_epochs(ResShared &sh, const ResPlaces<PT, PA
 // start, sums and stopping rule); leaves λ, the iteration count and any error in the pi_
 // fields and error of *st. part: one double per tile of A'ᵀ.
 template <int NC, bool ES, int PT, int PA>
-__device__ __noinline__ void res_power(ResShared &sh, const ResPlaces<PT, PA> &L, unsigned long long max_iters,
+__device__ __noinline__ void res_power(ResShared<uint16_t> &sh, const ResPlaces<PT, PA> &L, unsigned long long max_iters,
                                        double *part) {
-    constexpr bool CL = NC > 1;
-    const ResCtx &R = sh.R;
+    const ResCtx<uint16_t> &R = sh.R;
     const int n = R.T.rows, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     for (int k = threadIdx.x; k < n; k += RES_BT) dsm_at<double>(L.xbar + 8 * k) = 1.0 + 0.01 * (double)(R.T.perm[k] % 7);
     double s[1] = {0.0};
@@ -1077,7 +1132,7 @@ __device__ __noinline__ void res_power(ResShared &sh, const ResPlaces<PT, PA> &L
     const int a0 = (&dsm_at<int>(L.wtA))[warp], a1 = (&dsm_at<int>(L.wtA))[warp + 1];
     double *const contrib = R.contrib;
     const uint16_t *const perm = R.T.perm + R.T.p0;
-    res_sync<CL>();
+    res_sync<NC>();
     while (!done) {
         // tmp = A'(v·scale): the gathered vector is v after the scaling
         for (int k = threadIdx.x; k < n; k += RES_BT) dsm_at<double>(L.xbar + 8 * k) *= scale;
@@ -1092,7 +1147,7 @@ __device__ __noinline__ void res_power(ResShared &sh, const ResPlaces<PT, PA> &L
                 peers.put(at, a);
             }
         }
-        res_sync<CL>();
+        res_sync<NC>();
         // v = A'ᵀ tmp, with ‖v‖²
 #pragma unroll 1
         for (int ti = t0; ti < t1; ++ti) {
@@ -1105,9 +1160,9 @@ __device__ __noinline__ void res_power(ResShared &sh, const ResPlaces<PT, PA> &L
                 contrib[perm[k]] = 0.0 + a * a;
             }
         }
-        res_sync<CL>();
-        res_fold<CL, 1>(R.T, contrib, part, sh.sh);
-        res_sync<CL>();
+        res_sync<NC>();
+        res_fold<NC, 1>(R.T, contrib, part, sh.sh);
+        res_sync<NC>();
         res_total<1>(part, R.T.ntiles, s, sh.sh);
         const double norm = sqrt(s[0]);
         if (isnan(norm) || norm <= 0.0 || isinf(norm)) {
@@ -1140,7 +1195,7 @@ using ResSolverPlaces = ResPlaces<RES_PT, RES_PA>;
 // What the kernels of a solver need. `g` holds the solver's vectors in row order.
 struct ResArgs {
     SolverPtrs g;
-    ResSrc A, T;
+    ResSrc<uint16_t> A, T;
     ResVecs vec;
     double *contrib;                // [8n + 8m + 5n]
     double *ppart;
@@ -1149,7 +1204,7 @@ struct ResArgs {
     int mixed;
 };
 
-__host__ __device__ inline ResSolverPlaces res_solver_places(const ResSrc &A, const ResSrc &T, bool lo, bool entries) {
+__host__ __device__ inline ResSolverPlaces res_solver_places(const ResSrc<uint16_t> &A, const ResSrc<uint16_t> &T, bool lo, bool entries) {
     return ResSolverPlaces(A.rows, T.rows, lo, A.most_tasks, T.most_tasks, A.most_slots, T.most_slots, entries,
                            lo ? 4 : 8);
 }
@@ -1162,11 +1217,10 @@ struct ResNoStop {
 // form the FP64 kernel follows the FP32 one, and the one that is not due returns at once.
 template <int NC, bool LO, bool ES>
 __global__ void __launch_bounds__(RES_BT, 1) k_res_epochs(const __grid_constant__ ResArgs a, unsigned long long until) {
-    constexpr bool CL = NC > 1;
-    __shared__ ResShared s;
+    __shared__ ResShared<uint16_t> s;
     // the same for every CTA: the state is written after the last barrier
     if (a.g.st->done || a.g.st->total >= until || LO != (a.mixed && !a.g.st->fp64)) return;
-    const int c = CL ? (int)cluster_rank() : 0;
+    const int c = res_rank<NC>();
     if (threadIdx.x == 0) {
         s.st = *a.g.st;
         s.prm = *a.g.prm;
@@ -1178,7 +1232,7 @@ __global__ void __launch_bounds__(RES_BT, 1) k_res_epochs(const __grid_constant_
     }
     const ResSolverPlaces L = res_solver_places(a.A, a.T, LO, ES);
     res_open(s, L, a.A, a.T, a.g, a.vec, a.contrib, c);
-    const ResCtx &R = s.R;
+    const ResCtx<uint16_t> &R = s.R;
     const SolverPtrs &S = R.S, &g = a.g;
     if constexpr (ES) {
         if constexpr (LO) {
@@ -1212,9 +1266,9 @@ __global__ void __launch_bounds__(RES_BT, 1) k_res_epochs(const __grid_constant_
         S.y[k] = v;
         if (LO) S.y32[k] = (float)v;
     }
-    res_sync<CL>();
+    res_sync<NC>();
     res_epochs<NC, LO, ES>(s, L, ResNoStop{});
-    res_sync<CL>();
+    res_sync<NC>();
     for (int k = R.T.p0 + threadIdx.x; k < R.T.p1; k += RES_BT) {
         const int j = R.T.perm[k];
         g.x[j] = S.x[k];
@@ -1235,16 +1289,15 @@ __global__ void __launch_bounds__(RES_BT, 1) k_res_epochs(const __grid_constant_
 // The solver's power iteration.
 template <int NC, bool ES>
 __global__ void __launch_bounds__(RES_BT, 1) k_res_power(const __grid_constant__ ResArgs a, unsigned long long max_iters) {
-    __shared__ ResShared s;
-    constexpr bool CL = NC > 1;
-    const int c = CL ? (int)cluster_rank() : 0;
+    __shared__ ResShared<uint16_t> s;
+    const int c = res_rank<NC>();
     const ResSolverPlaces L = res_solver_places(a.A, a.T, false, ES);
     res_open(s, L, a.A, a.T, a.g, a.vec, a.contrib, c);
     if constexpr (ES) {
         res_load_entries<double>(s.R.A, s.R.A.v, L.valA, L.atA, L.xbar);
         res_load_entries<double>(s.R.T, s.R.T.v, L.valT, L.atT, L.y);
     }
-    res_sync<CL>();
+    res_sync<NC>();
     res_power<NC, ES>(s, L, max_iters, a.ppart);
     if (c == 0 && threadIdx.x == 0) {
         a.g.st->pi_scale = s.st.pi_scale;
@@ -1255,19 +1308,33 @@ __global__ void __launch_bounds__(RES_BT, 1) k_res_power(const __grid_constant__
     }
 }
 
+// The CTA of task ti: the last whose first task is at most ti.
+template <class IX>
+__device__ __forceinline__ int res_cta_of(const ResSrc<IX> &M, int ti, int ctas) {
+    int c = 0;
+    for (int hi = ctas; hi - c > 1;) {
+        const int mid = (c + hi) / 2;
+        if (M.wt[mid * RES_W] <= ti) c = mid;
+        else hi = mid;
+    }
+    return c;
+}
+
 // The slots of one matrix from its CSR arrays, one warp per task: columns renamed to the
-// positions of the other matrix's rows; padding holds -0.0 and the position past them.
-static __global__ void __launch_bounds__(NT) k_res_fill(ResSrc M, int ctas, int ntasks, int other_rows,
-                                                        const uint16_t *__restrict__ other_inv,
-                                                        const int *__restrict__ ci, const double *__restrict__ v) {
+// positions of the other matrix's rows; padding holds -0.0 and a position past them (`spread`
+// such positions of which 0, 4, 8, ... are used, task by task).
+template <class IX>
+__global__ void __launch_bounds__(NT) k_res_fill(ResSrc<IX> M, int ctas, int ntasks, int other_rows, int spread,
+                                                 const IX *__restrict__ other_inv, const int *__restrict__ ci,
+                                                 const double *__restrict__ v) {
     const int lane = threadIdx.x & 31;
     for (int ti = (blockIdx.x * NT + threadIdx.x) >> 5; ti < ntasks; ti += gridDim.x * (NT / 32)) {
-        int c = 0;
-        while (c + 1 < ctas && M.wt[(c + 1) * RES_W] <= ti) ++c;
+        const int c = res_cta_of(M, ti, ctas);
         const ResTask t = M.tasks[ti];
+        const IX none = (IX)(other_rows + 4 * ti % spread);
         auto put = [&](int d, int k, bool in) {
             const double x = in ? v[k] : -0.0;
-            M.ci[d] = in ? other_inv[ci[k]] : (uint16_t)other_rows;
+            M.ci[d] = in ? other_inv[ci[k]] : none;
             M.v[d] = x;
             if (M.v32) M.v32[d] = (float)x;
         };

@@ -219,6 +219,7 @@ extern "C" int sp_server_create(sp_ctx *ctx, const sp_server_config *cfg, const 
             sp_server_destroy(s);
             return rc;
         }
+        c->shared = true;
         s->slot_ctx.push_back(c);
     }
     int rc = sp_ctx_create(ctx->device, &s->batch_ctx);

@@ -941,10 +941,19 @@ void launch_sell(sp_solver *s, const SellMat &S, cudaStream_t st, const Op &op) 
 // A problem under SMALL_NNZ nonzeros keeps both passes on the tile engine: there an
 // iteration's time is launch latency and tile parallelism (32 LPs of the batch workload,
 // one device solve each: 9.1 µs per iteration on tiles, 9.5 stream, 11.6 SELL).
+// Where an epoch engine runs the MID passes (res_build, GridPlan), these are what it leaves and
+// what direct, timed launches use.
 // SP_PASS_ENGINE=tiles|stream|sell overrides all four (large: the assignment above for a
-// problem of any size), SP_PRIMAL_ENGINE and SP_DUAL_ENGINE one pass; SP_STREAM_GATHER
+// problem of any size; resident, grid: the epoch engine, at any size that it can hold),
+// SP_PRIMAL_ENGINE and SP_DUAL_ENGINE one pass; SP_STREAM_GATHER
 // names the stream variant.
 constexpr int64_t SMALL_NNZ = 1 << 20;
+
+// Whether the environment asks for engines other than the epoch engine `mine`.
+bool other_engine_asked(const char *mine) {
+    const char *eng = getenv("SP_PASS_ENGINE");
+    return (eng && strcmp(eng, mine)) || getenv("SP_PRIMAL_ENGINE") || getenv("SP_DUAL_ENGINE");
+}
 
 int choose_engines(sp_solver *s) {
     const char *eng = getenv("SP_PASS_ENGINE");
@@ -1008,7 +1017,7 @@ int choose_engines(sp_solver *s) {
 // ------------------------------------------------------------------ the on-chip engine
 
 constexpr int RES_SMEM_MAX = (int)STREAM_SMEM_MAX - 4096;  // dynamic shared memory of a CTA, beside ResShared
-static_assert(sizeof(ResShared) <= 4096, "the static part fits beside it");
+static_assert(sizeof(ResShared<uint16_t>) <= 4096, "the static part fits beside it");
 constexpr uint64_t RES_MAX_EPOCHS = 16;  // epochs of one launch at most
 
 template <int NC>
@@ -1057,17 +1066,16 @@ int res_cluster_of(int64_t m, int64_t n, int64_t nnz) {
 // tile, and its vectors in the CTAs' shared memory. rp_t: the row pointers of A'ᵀ.
 int res_build(sp_solver *s, const sp_lp *lp, const std::vector<int> &rp_t) {
     const int64_t m = s->m, n = s->n, nnz = s->nnz;
-    const char *eng = getenv("SP_PASS_ENGINE");
-    if (eng && strcmp(eng, "resident")) return SP_OK;  // another engine is asked for
+    if (other_engine_asked("resident")) return SP_OK;
     if (nnz >= SMALL_NNZ || nnz == 0 || m > RES_MAX_ROWS || n > RES_MAX_ROWS || m < 1 || n < 1) return SP_OK;
     const int ctas = res_cluster_of(m, n, nnz);
     if (s->A.nlong || s->AT.nlong || m > (int64_t)RES_PA * ctas || n > (int64_t)RES_PT * ctas) return SP_OK;
     ResPlan PA, PT;
-    res_plan(lp->a.row_ptr, (int)m, ctas, &PA);
-    res_plan(rp_t.data(), (int)n, ctas, &PT);
+    res_plan(lp->a.row_ptr, (int)m, ctas, true, &PA);
+    res_plan(rp_t.data(), (int)n, ctas, true, &PT);
     if (PA.most_rows > RES_PA || PT.most_rows > RES_PT) return SP_OK;
     ResArgs &a = s->res;
-    auto sizes = [](ResSrc &q, const ResPlan &P, const DevCsr &M) {
+    auto sizes = [](ResSrc<uint16_t> &q, const ResPlan &P, const DevCsr &M) {
         q.rows = (int)M.nrows;
         q.heavy = P.heavy;
         q.ntiles = M.ntiles;
@@ -1135,7 +1143,7 @@ int res_build(sp_solver *s, const sp_lp *lp, const std::vector<int> &rp_t) {
     if ((rc = dmalloc(&s->res_mem, bytes))) return rc;
     unsigned char *d = (unsigned char *)s->res_mem;
     SP_CUDA_TRY(cudaMemcpyAsync(d, h.data(), up, cudaMemcpyHostToDevice, st));
-    auto place = [&](ResSrc &q, const Off &o) {
+    auto place = [&](ResSrc<uint16_t> &q, const Off &o) {
         q.tasks = (const ResTask *)(d + o.tasks);
         q.wt = (const int *)(d + o.wt);
         q.p0 = (const int *)(d + o.p0);
@@ -1156,11 +1164,282 @@ int res_build(sp_solver *s, const sp_lp *lp, const std::vector<int> &rp_t) {
     a.mixed = s->mixed;
     a.g = ptrs_of(s);
     const int ta = (int)PA.tasks.size(), tt = (int)PT.tasks.size(), W = NT / 32;
-    k_res_fill<<<(ta + W - 1) / W, NT, 0, st>>>(a.A, ctas, ta, (int)n, (const uint16_t *)(d + ot.inv), s->A.ci, s->A.v);
-    k_res_fill<<<(tt + W - 1) / W, NT, 0, st>>>(a.T, ctas, tt, (int)m, (const uint16_t *)(d + oa.inv), s->AT.ci, s->AT.v);
+    k_res_fill<<<(ta + W - 1) / W, NT, 0, st>>>(a.A, ctas, ta, (int)n, 1, (const uint16_t *)(d + ot.inv), s->A.ci, s->A.v);
+    k_res_fill<<<(tt + W - 1) / W, NT, 0, st>>>(a.T, ctas, tt, (int)m, 1, (const uint16_t *)(d + oa.inv), s->AT.ci, s->AT.v);
     SP_CUDA_TRY(cudaGetLastError());
     SP_CUDA_TRY(cudaStreamSynchronize(st));  // the host's copy of the plans ends here
     s->res_ctas = ctas;
+    return SP_OK;
+}
+
+// Calls body(w, k0, k1) for up to 16 contiguous ranges [k0, k1) of [0, len), each on a host
+// thread of its own when there is more than one.
+template <class F>
+void split_ranges(int64_t len, const F &body) {
+    const int workers = (int)std::max<int64_t>(1, std::min<int64_t>(16, len >> 18));
+    if (workers == 1) {
+        body(0, 0, len);
+        return;
+    }
+    std::vector<std::thread> th;
+    for (int w = 0; w < workers; ++w) th.emplace_back(body, w, len * w / workers, len * (w + 1) / workers);
+    for (auto &t : th) t.join();
+}
+
+// ------------------------------------------------------------------ the grid engine
+
+constexpr int GRID_PT = 1024, GRID_PA = 512;     // columns and rows of a CTA with entries in shared memory
+constexpr int GRID_PT2 = 2560, GRID_PA2 = 1280;  // ... without
+
+int grid_launch(const sp_solver *s, const GridLaunch &l, int n) {
+    cudaStream_t st = s->ctx->stream;
+    SP_CUDA_TRY(cudaMemsetAsync(s->grid.bar, 0, sizeof(GridBar), st));
+    void *args[] = {(void *)&s->grid, (void *)&n};
+    SP_CUDA_TRY(cudaLaunchCooperativeKernel((const void *)l.f, dim3((unsigned)s->grid_ctas), dim3(RES_BT), args,
+                                            (size_t)l.smem, st));
+    return SP_OK;
+}
+
+// Sort keys of the rows: longest first.
+__global__ void k_grid_keys(const int *__restrict__ rp, int64_t rows, uint16_t *__restrict__ key, int *__restrict__ row) {
+    GRID_LOOP(r, rows) {
+        key[r] = (uint16_t)(TILE_NNZ - (rp[r + 1] - rp[r]));
+        row[r] = (int)r;
+    }
+}
+// The rows of each task, from the rows in the order of decreasing length; one warp per task.
+__global__ void k_grid_perm(ResSrc<int> M, const int *__restrict__ first, const int *__restrict__ order, int ctas,
+                            int *__restrict__ perm, int *__restrict__ inv) {
+    const int lane = threadIdx.x & 31, ntasks = M.wt[ctas * RES_W];
+    for (int ti = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; ti < ntasks; ti += (gridDim.x * blockDim.x) >> 5) {
+        const int c = res_cta_of(M, ti, ctas);
+        const ResTask t = M.tasks[ti];
+        if (lane < t.z) {
+            const int p = M.p0[c] + t.y + lane, r = order[first[ti] + lane];
+            perm[p] = r;
+            inv[r] = p;
+        }
+    }
+}
+
+// Which row is at which position of a planned matrix: a stable radix sort by length (ties in
+// row order, as res_plan's), then the tasks' rows.
+int grid_order(sp_solver *s, const DevCsr &D, const ResSrc<int> &M, const int *first, int ctas, int *perm, int *inv) {
+    cudaStream_t st = s->ctx->stream;
+    const int64_t rows = D.nrows;
+    uint16_t *key = nullptr, *skey = nullptr;
+    int *row = nullptr, *order = nullptr;
+    void *tmp = nullptr;
+    size_t bytes = 0;
+    auto done = [&](int rc) {
+        for (void *p : {(void *)key, (void *)skey, (void *)row, (void *)order, tmp}) dfree(p, st);
+        return rc;
+    };
+    int rc;
+    if ((rc = dalloc(&key, rows)) || (rc = dalloc(&skey, rows)) || (rc = dalloc(&row, rows)) || (rc = dalloc(&order, rows)))
+        return done(rc);
+    k_grid_keys<<<grid_of(s->ctx, rows), NT, 0, st>>>(D.rp, rows, key, row);
+    constexpr int bits = 12;  // lengths up to TILE_NNZ
+    static_assert(TILE_NNZ < (1 << bits), "a length fits its key");
+    cudaError_t e = cub::DeviceRadixSort::SortPairs(nullptr, bytes, key, skey, row, order, (int)rows, 0, bits, st);
+    if (e == cudaSuccess && (rc = dmalloc(&tmp, bytes))) return done(rc);
+    if (e == cudaSuccess) e = cub::DeviceRadixSort::SortPairs(tmp, bytes, key, skey, row, order, (int)rows, 0, bits, st);
+    if (e != cudaSuccess) return done(fail(SP_ERR_CUDA, std::string("grid engine's order: ") + cudaGetErrorString(e)));
+    k_grid_perm<<<grid_of(s->ctx, rows), NT, 0, st>>>(M, first, order, ctas, perm, inv);
+    return done(SP_OK);
+}
+
+// The cuts of both matrices, made on a host thread beside the scaling sweeps, for an LP in the
+// grid engine's range: no row longer than a tile, and alone on the device as far as this
+// library knows (a context that solves beside others keeps to launches, which share the SMs).
+//
+// µs an iteration, launches | grid (FP64): random 80k nonzeros 10.4 | 7.4, 200k 10.5 | 8.5,
+// 2M 36.1 | 28.7, 12M 168 | 144, 16M 222 | 191; power law 60k 11.3 | 11.2, 500k 15.1 | 13.0,
+// 3M 47.0 | 40.8, 10M 128 | 107, 22M 253 | 239, 40M 446 | 434 for 100 ms more of set-up: hence
+// GRID_MAX_NNZ. Transport, whose gathers are consecutive or of a small vector, so that the
+// stream engine's wide loads count: 500k 11.3 | 10.9, 1.6M 36.9 | 26.6, 3.4M 51.9 | 52.9, 8M
+// 113 | 115 (mixed 3.4M 43.7 | 51.3): hence GRID_MAX_LONG for rows of GRID_LONG_ROW on average.
+//
+// The power iteration (ms, launches | grid): 80k 0.88 | 0.48, 200k 3.67 | 2.20, 500k 3.62 | 2.18,
+// 1M 5.35 | 3.80, 2M 5.06 | 4.48, 3M 10.3 | 10.6. From 1M on the norms' chains of additions,
+// which hold SMs beside it that the grid has to wait for, count: hence GRID_POWER_MAX_NNZ.
+constexpr int64_t GRID_MAX_NNZ = 3 << 23, GRID_MAX_LONG = 1 << 21, GRID_LONG_ROW = 128, GRID_POWER_MAX_NNZ = 1 << 19;
+struct GridPlan {
+    std::thread th;
+    ResCuts A, T;
+    int ctas = 0;
+    bool ok = false;
+    ~GridPlan() { join(); }
+    bool join() {
+        if (th.joinable()) th.join();
+        return ok;
+    }
+    // rp_t: the row pointers of A'ᵀ. Both arrays of row pointers live until join().
+    int start(const sp_solver *s, const sp_lp *lp, const std::vector<int> &rp_t) {
+        const int64_t m = s->m, n = s->n, nnz = s->nnz;
+        if (other_engine_asked("grid")) return SP_OK;
+        const bool forced = getenv("SP_PASS_ENGINE") != nullptr;
+        if (nnz < 1 || m < 1 || n < 1 || s->A.nlong) return SP_OK;
+        if (!forced && (s->ctx->shared || nnz > GRID_MAX_NNZ || (nnz > GRID_MAX_LONG && nnz / m >= GRID_LONG_ROW)))
+            return SP_OK;
+        int coop = 0;
+        SP_CUDA_TRY(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, s->ctx->device));
+        if (!coop) return SP_OK;
+        ctas = (int)std::min<int64_t>(s->ctx->sms, std::max<int64_t>(4, nnz / 1000));
+        const int64_t *rp_a = lp->a.row_ptr;
+        const int *rpt = rp_t.data();
+        auto cut = [this](auto rp, int64_t rows, ResCuts *P) {
+            std::vector<int> count(TILE_NNZ + 1, 0);
+            for (int64_t r = 0; r < rows; ++r) {
+                const int64_t len = (int64_t)(rp[r + 1] - rp[r]);
+                if (len > TILE_NNZ) return false;
+                ++count[(size_t)len];
+            }
+            res_cut(count, ctas, false, P);
+            return true;
+        };
+        try {
+            th = std::thread([=] {
+                try {
+                    ok = cut(rp_a, m, &A) && cut(rpt, n, &T);
+                } catch (const std::exception &) {  // no memory for it: the launched engines serve
+                }
+            });
+        } catch (const std::exception &) {  // no thread for it
+        }
+        return SP_OK;
+    }
+};
+
+// Sets the grid engine up from its plan.
+int grid_build(sp_solver *s, GridPlan &plan_of) {
+    if (s->res_ctas || !plan_of.join()) return SP_OK;
+    const int64_t m = s->m, n = s->n;
+    const int ctas = plan_of.ctas;
+    const ResCuts &PA = plan_of.A, &PT = plan_of.T;
+    GridArgs &a = s->grid;
+    auto sizes = [](ResSrc<int> &q, const ResCuts &P, const DevCsr &M) {
+        q.rows = (int)M.nrows;
+        q.heavy = P.heavy;
+        q.ntiles = M.ntiles;
+        q.most_rows = P.most_rows;
+        q.most_slots = P.most_slots;
+        q.most_tasks = P.most_tasks;
+        q.rp = M.rp;
+        q.tiles = M.tiles;
+    };
+    sizes(a.A, PA, s->A);
+    sizes(a.T, PT, s->AT);
+    // what fits in shared memory: row inputs and entries, row inputs, or neither
+    for (int lo = 0; lo < (s->mixed ? 2 : 1); ++lo) {
+        GridLaunch &l = s->grid_mid[lo];
+        const int both = grid_places<true, true, GRID_PT, GRID_PA>(a, lo).total;
+        const int rows = grid_places<true, false, GRID_PT2, GRID_PA2>(a, lo).total;
+        const int none = grid_places<false, false, 0, 0>(a, lo).total;
+        if (PT.most_rows <= GRID_PT && PA.most_rows <= GRID_PA && both <= RES_SMEM_MAX)
+            l = {lo ? k_grid_mid<true, true, true, GRID_PT, GRID_PA> : k_grid_mid<false, true, true, GRID_PT, GRID_PA>, both};
+        else if (PT.most_rows <= GRID_PT2 && PA.most_rows <= GRID_PA2 && rows <= RES_SMEM_MAX)
+            l = {lo ? k_grid_mid<true, true, false, GRID_PT2, GRID_PA2> : k_grid_mid<false, true, false, GRID_PT2, GRID_PA2>, rows};
+        else if (none <= RES_SMEM_MAX)
+            l = {lo ? k_grid_mid<true, false, false, 0, 0> : k_grid_mid<false, false, false, 0, 0>, none};
+        else
+            return SP_OK;
+        if (lo == 0 && s->nnz <= GRID_POWER_MAX_NNZ) {  // the power iteration has no row inputs
+            const int pe = grid_places<false, true, 0, 0>(a, false).total, pn = grid_places<false, false, 0, 0>(a, false).total;
+            s->grid_power = pe <= RES_SMEM_MAX ? GridLaunch{k_grid_power<true>, pe} : GridLaunch{k_grid_power<false>, pn};
+        }
+    }
+    for (const GridLaunch *l : {&s->grid_mid[0], &s->grid_mid[1], &s->grid_power}) {
+        if (!l->f) continue;
+        SP_CUDA_TRY(cudaFuncSetAttribute((const void *)l->f, cudaFuncAttributeMaxDynamicSharedMemorySize, RES_SMEM_MAX));
+        int per_sm = 0;
+        SP_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, (const void *)l->f, RES_BT, (size_t)l->smem));
+        if ((int64_t)per_sm * s->ctx->sms < ctas) return SP_OK;
+    }
+    // one allocation: the plans, the slots and the position-space vectors
+    size_t bytes = 0;
+    auto room = [&](size_t b) {
+        const size_t at = bytes;
+        bytes += (b + 255) & ~size_t(255);
+        return at;
+    };
+    std::vector<std::pair<size_t, std::pair<const void *, size_t>>> ups;
+    auto vec = [&](const auto &v) {
+        const size_t b = v.size() * sizeof(v[0]), at = room(b);
+        if (b) ups.push_back({at, {v.data(), b}});
+        return at;
+    };
+    struct Off {
+        size_t perm, inv, tasks, first, wt, p0, s0, ci, v, v32;
+    } oa{}, ot{};
+    auto plan = [&](const ResCuts &P, const DevCsr &M, Off *o) {
+        o->perm = room(sizeof(int) * (size_t)M.nrows);
+        o->inv = room(sizeof(int) * (size_t)M.nrows);
+        o->tasks = vec(P.tasks);
+        o->first = vec(P.first);
+        o->wt = vec(P.wt);
+        o->p0 = vec(P.p0);
+        o->s0 = vec(P.s0);
+        o->ci = room(sizeof(int) * (size_t)P.slots);
+        o->v = room(sizeof(double) * (size_t)P.slots);
+        o->v32 = s->mixed ? room(sizeof(float) * (size_t)P.slots) : 0;
+    };
+    plan(PA, s->A, &oa);
+    plan(PT, s->AT, &ot);
+    const size_t N = (size_t)n, M = (size_t)m;
+    const size_t inputs = room(8 * (5 * N + 3 * M)), gathered = room(8 * (N + M + 2 * GRID_ONES));
+    const size_t gathered32 = s->mixed ? room(4 * (N + M + 2 * GRID_ONES)) : 0;
+    const size_t contrib = room(8 * N), bar = room(sizeof(GridBar));
+    cudaStream_t st = s->ctx->stream;
+    int rc;
+    if (dmalloc(&s->res_mem, bytes)) {  // no room for it: the launched engines need none
+        s->ctx->last_error.clear();
+        return SP_OK;
+    }
+    unsigned char *d = (unsigned char *)s->res_mem;
+    for (const auto &u : ups) SP_CUDA_TRY(cudaMemcpyAsync(d + u.first, u.second.first, u.second.second, cudaMemcpyHostToDevice, st));
+    auto place = [&](ResSrc<int> &q, const Off &o) {
+        q.tasks = (const ResTask *)(d + o.tasks);
+        q.wt = (const int *)(d + o.wt);
+        q.p0 = (const int *)(d + o.p0);
+        q.s0 = (const int *)(d + o.s0);
+        q.perm = (const int *)(d + o.perm);
+        q.ci = (int *)(d + o.ci);
+        q.v = (double *)(d + o.v);
+        q.v32 = s->mixed ? (float *)(d + o.v32) : nullptr;
+    };
+    place(a.A, oa);
+    place(a.T, ot);
+    double *v = (double *)(d + inputs);
+    for (double **q : {&a.x, &a.c, &a.lv, &a.uv, &a.xa}) {
+        *q = v;
+        v += N;
+    }
+    for (double **q : {&a.lc, &a.uc, &a.ya}) {
+        *q = v;
+        v += M;
+    }
+    a.y = (double *)(d + gathered);
+    a.xbar = a.y + M + GRID_ONES;
+    a.y32 = s->mixed ? (float *)(d + gathered32) : nullptr;
+    a.xbar32 = s->mixed ? a.y32 + M + GRID_ONES : nullptr;
+    a.contrib = (double *)(d + contrib);
+    a.bar = (GridBar *)(d + bar);
+    a.ppart = s->ppart;
+    a.mixed = s->mixed;
+    a.g = ptrs_of(s);
+    k_grid_ones<<<GRID_ONES / NT, NT, 0, st>>>(a);
+    if ((rc = grid_order(s, s->A, a.A, (const int *)(d + oa.first), ctas, (int *)(d + oa.perm), (int *)(d + oa.inv))) ||
+        (rc = grid_order(s, s->AT, a.T, (const int *)(d + ot.first), ctas, (int *)(d + ot.perm), (int *)(d + ot.inv)))) {
+        cudaStreamSynchronize(st);
+        return rc;
+    }
+    const int ta = (int)PA.tasks.size(), tt = (int)PT.tasks.size(), W = NT / 32, most = s->ctx->sms * 16;
+    k_res_fill<int><<<std::min(most, (ta + W - 1) / W), NT, 0, st>>>(a.A, ctas, ta, (int)n, GRID_ONES, (const int *)(d + ot.inv), s->A.ci, s->A.v);
+    k_res_fill<int><<<std::min(most, (tt + W - 1) / W), NT, 0, st>>>(a.T, ctas, tt, (int)m, GRID_ONES, (const int *)(d + oa.inv), s->AT.ci, s->AT.v);
+    SP_CUDA_TRY(cudaGetLastError());
+    SP_CUDA_TRY(cudaStreamSynchronize(st));  // the host's copy of the plans ends here
+    s->grid_ctas = ctas;  // the inputs follow once the scaled vectors are final (grid_inputs)
     return SP_OK;
 }
 
@@ -1280,12 +1559,19 @@ void launch_T(sp_solver *s, int i, cudaStream_t st) {
 
 // One epoch of E iterations (the last is the check) on stream `st`. With timing
 // on, CUDA events bracket the P and D launches of sampled MID iterations.
-void enqueue_epoch(sp_solver *s, int E, cudaStream_t st, bool timed) {
+int enqueue_epoch(sp_solver *s, int E, cudaStream_t st, bool timed) {
+    int rc = SP_OK;
     const SolverPtrs p = ptrs_of(s);
     const int gn = grid_of(s->ctx, std::max(s->n, s->m));
     for (int i = 0; i < E; ++i) {
         const bool last = i == E - 1;
         const int role = last ? ROLE_CHECK : (i == 0 ? ROLE_FIRST : ROLE_MID);
+        if (role == ROLE_MID && s->grid_ctas && !timed) {  // all MID iterations at once
+            if (!rc && s->mixed) rc = grid_launch(s, s->grid_mid[1], E);
+            if (!rc) rc = grid_launch(s, s->grid_mid[0], E);
+            i = E - 2;
+            continue;
+        }
         bool sample = timed && role == ROLE_MID && s->timing_every > 0 && (s->timing_counter++ % s->timing_every == 0);
         cudaEvent_t e0 = nullptr, e1 = nullptr, e2 = nullptr;
         if (sample) {
@@ -1311,6 +1597,7 @@ void enqueue_epoch(sp_solver *s, int E, cudaStream_t st, bool timed) {
             k_finish<<<gn, NT, 0, st>>>(p, s->n, s->m);
         }
     }
+    return rc;
 }
 
 int set_smem_limits() {
@@ -1332,8 +1619,12 @@ int build_graph(sp_solver *s, int E, cudaGraphExec_t *out) {
     cudaStream_t st = s->ctx->stream;
     cudaGraph_t g;
     SP_CUDA_TRY(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
-    enqueue_epoch(s, E, st, false);
+    const int rc = enqueue_epoch(s, E, st, false);
     SP_CUDA_TRY(cudaStreamEndCapture(st, &g));
+    if (rc) {
+        cudaGraphDestroy(g);
+        return rc;
+    }
     // the epoch's kernel launches, for the callers that count them
     size_t nodes = 0;
     int64_t kernels = 0;
@@ -1701,20 +1992,6 @@ std::string rust_display(double v) {
     return out;
 }
 
-// Calls body(w, k0, k1) for up to 16 contiguous ranges [k0, k1) of [0, len), each on a host
-// thread of its own when there is more than one.
-template <class F>
-void split_ranges(int64_t len, const F &body) {
-    const int workers = (int)std::max<int64_t>(1, std::min<int64_t>(16, len >> 18));
-    if (workers == 1) {
-        body(0, 0, len);
-        return;
-    }
-    std::vector<std::thread> th;
-    for (int w = 0; w < workers; ++w) th.emplace_back(body, w, len * w / workers, len * (w + 1) / workers);
-    for (auto &t : th) t.join();
-}
-
 // LpProblem::validate (problem.rs:166-194), its checks in its order and with its messages
 // (SP_ERR_PROBLEM): the variables' bounds (NaN, then crossed) over all columns, then the
 // constraints', then NaN among the coefficients c and then A's values (numbered after c).
@@ -1798,13 +2075,16 @@ int validate_lp(const sp_lp *lp) {
     return rc ? fail(rc, msg) : SP_OK;
 }
 
+constexpr const char *GRID_STALL_MESSAGE = "the grid's barrier did not complete within its wait limit";
+
 int power_iteration(sp_solver *s) {  // Solver::estimate_norm (solver.rs:215-242)
     cudaStream_t st = s->ctx->stream;
     if (s->n == 0 || s->nnz == 0) {
         s->norm_est = 1.0;
         return SP_OK;
     }
-    if (!s->res_ctas) {
+    const bool once = s->res_ctas || (s->grid_ctas && s->grid_power.f);  // all iterations in one launch
+    if (!once) {
         k_power_fill<<<grid_of(s->ctx, s->n), NT, 0, st>>>(s->pv, s->n);
         k_power_init<<<1, NT, 0, st>>>(s->n, s->ppart);
         k_power_start<<<1, 32, 0, st>>>(s->ppart, s->d_st);
@@ -1813,14 +2093,17 @@ int power_iteration(sp_solver *s) {  // Solver::estimate_norm (solver.rs:215-242
     PowerA a{s->A.rp, s->A.ci, s->A.v, s->A.tiles, s->pv, s->ptmp, s->d_st, 0.0};
     PowerT t{s->AT.rp, s->AT.ci, s->AT.v, s->AT.tiles, s->ptmp, s->pv, s->ppart, s->d_st};
     const uint64_t chunk = 8;
-    if (s->res_ctas && maxit > 0) {  // a small LP: all iterations in one launch
-        const int rc = res_launch(s, s->res_power, maxit);
+    if (once && maxit > 0) {
+        // pi_done tells a finished iteration from a stalled one: no error is left from before
+        SP_CUDA_TRY(cudaMemsetAsync(s->d_st, 0, sizeof(DevState), st));
+        const int rc = s->res_ctas ? res_launch(s, s->res_power, maxit)
+                                   : grid_launch(s, s->grid_power, (int)std::min<uint64_t>(maxit, INT32_MAX));
         if (rc) return rc;
     }
     DevState h{};  // with no iterations, λ stays 0 as in the reference
     for (uint64_t done_it = 0; done_it < maxit;) {
-        const uint64_t c = s->res_ctas ? maxit : std::min(chunk, maxit - done_it);
-        for (uint64_t q = 0; q < c && !s->res_ctas; ++q) {
+        const uint64_t c = once ? maxit : std::min(chunk, maxit - done_it);
+        for (uint64_t q = 0; q < c && !once; ++q) {
             // A'·v on the SELL copy where the dual passes have one (the same bits; 0.21 ms on
             // the tile engine for the 40M LP), else on the tile engine
             if (s->sellA.ok) launch_sell(s, s->sellA, st, a);
@@ -1833,6 +2116,7 @@ int power_iteration(sp_solver *s) {  // Solver::estimate_norm (solver.rs:215-242
         SP_CUDA_TRY(cudaStreamSynchronize(st));
         if (h.pi_done) break;
     }
+    if (h.error == ERR_GRID_STALL) return fail(SP_ERR_CUDA, GRID_STALL_MESSAGE);
     if (h.error == ERR_NUMERICAL_POWER) return fail(SP_ERR_NUMERICAL, "numerical breakdown: power iteration collapsed");
     s->norm_est = sqrt(h.pi_lambda) * 1.01;  // solver.rs:241
     s->pi_iters = h.pi_iters;
@@ -1974,6 +2258,8 @@ extern "C" int sp_solver_create(sp_ctx *ctx, const sp_lp *lp, const sp_solver_pa
         (rc = dalloc(&s->row_scale, m)) || (rc = dalloc(&s->col_scale, n)) || (rc = dalloc(&s->scales, 2)) ||
         (rc = dalloc(&s->norms, 4)))
         return cleanup(rc);
+    GridPlan grid_plan;
+    if ((rc = grid_plan.start(s, lp, rp_t))) return cleanup(rc);
     if ((rc = scale_on_device(s, lp, rp_t, &side))) return cleanup(rc);
     // the host's tile plan of A'ᵀ while the GPU runs the scaling sweeps
     if ((rc = plan_transpose(s, rp_t))) return cleanup(rc);
@@ -2000,7 +2286,8 @@ extern "C" int sp_solver_create(sp_ctx *ctx, const sp_lp *lp, const sp_solver_pa
     SP_CUDA_TRY(cudaMallocHost(&s->h_st, sizeof(DevState) * (SolverLookahead + 2)));
     if ((rc = set_smem_limits())) return cleanup(rc);
     if ((rc = choose_engines(s))) return cleanup(rc);
-    if ((rc = res_build(s, lp, rp_t))) return cleanup(rc);
+    if ((rc = res_build(s, lp, rp_t)) || (rc = grid_build(s, grid_plan))) return cleanup(rc);
+    grid_plan.join();
     rp_t = std::vector<int>();
     stage("engines");
     // ‖A'‖₂ and η (solver.rs:316), while the second stream forms the norms
@@ -2011,6 +2298,10 @@ extern "C" int sp_solver_create(sp_ctx *ctx, const sp_lp *lp, const sp_solver_pa
     SP_CUDA_TRY(cudaMemcpyAsync(hn, s->norms, sizeof hn, cudaMemcpyDeviceToHost, ctx->stream));
     SP_CUDA_TRY(cudaMemcpyAsync(hs, s->scales, sizeof hs, cudaMemcpyDeviceToHost, ctx->stream));
     SP_CUDA_TRY(cudaStreamSynchronize(ctx->stream));
+    if (s->grid_ctas) {  // the scaled vectors are final
+        k_grid_inputs<<<grid_of(ctx, std::max(m, n)), NT, 0, ctx->stream>>>(s->grid);
+        SP_CUDA_TRY(cudaGetLastError());
+    }
     s->b_norm = hn[2];
     s->c_norm = hn[3];
     s->bound_scale = hs[0];
@@ -2093,7 +2384,8 @@ int launch_epoch(sp_solver *s, int E) {
     cudaStream_t st = s->ctx->stream;
     if (res_epochs_on(s)) return res_launch_next(s, 1);
     if (s->timing_every > 0) {
-        enqueue_epoch(s, E, st, true);
+        const int rc = enqueue_epoch(s, E, st, true);
+        if (rc) return rc;
     } else {
         cudaGraphExec_t g;
         int rc = epoch_graph(s, E, &g);
@@ -2221,6 +2513,7 @@ extern "C" int sp_solver_solve(sp_solver *s, sp_solution_info *info) {
     last = s->h_st[0];
     s->solve_s = now_s() - t0;
     if (last.error == ERR_NUMERICAL_ITERATES) return fail(SP_ERR_NUMERICAL, "numerical breakdown: iterates are not finite");
+    if (last.error == ERR_GRID_STALL) return fail(SP_ERR_CUDA, GRID_STALL_MESSAGE);
     if (last.error == ERR_PIPELINE_STALL)
         return fail(SP_ERR_CUDA, "a bulk copy of the pass pipeline did not complete within its wait limit");
     if (!last.done && !s->time_limited) s->time_limited = true;  // only reachable with an exhausted limit

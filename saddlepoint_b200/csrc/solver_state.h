@@ -5,6 +5,7 @@
 #include <vector>
 
 #include "internal.cuh"
+#include "grid.cuh"
 #include "resident.cuh"
 #include "sell.cuh"
 #include "stream.cuh"
@@ -14,6 +15,11 @@ constexpr int SolverLookahead = 2;  // epochs queued ahead of the state the host
 using ResKernel = void (*)(ResArgs, unsigned long long);
 struct ResLaunch {  // a kernel of the on-chip engine and its dynamic shared memory
     ResKernel f = nullptr;
+    int smem = 0;
+};
+using GridKernel = void (*)(GridArgs, int);
+struct GridLaunch {
+    GridKernel f = nullptr;
     int smem = 0;
 };
 struct TimingSample {
@@ -38,6 +44,10 @@ struct sp_solver {
     sp::ResArgs res{};
     sp::ResLaunch res_epochs[2], res_power;  // epochs in FP64 and of the FP32 phase
     void *res_mem = nullptr;
+    // a mid-sized LP's engine over the whole grid (grid.cuh; 0 CTAs: not used), its memory in res_mem
+    int grid_ctas = 0;
+    sp::GridArgs grid{};
+    sp::GridLaunch grid_mid[2], grid_power;  // an epoch's iterations in FP64 and in the FP32 phase
     double *contrib = nullptr;   // [NP_D][m] row contributions of the check's dual pass on the SELL copy
     int64_t m = 0, n = 0, nnz = 0;
     double c0 = 0.0;
