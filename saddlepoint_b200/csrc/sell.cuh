@@ -16,7 +16,8 @@
 // entries (the last one padded with column -1), the rows one after another in row order;
 // lane `lane` of a chunk holds entry lane + 32·chunk of its row. The chunks are cut into
 // blocks of SELL_SEG_CHUNKS; a warp takes the rows that start in one block — a segment, at
-// most SELL_SEG_CHUNKS / 2 rows since each has at least two chunks — (k_sell_rows) and
+// most SELL_SEG_CHUNKS / 2 rows since each has at least two chunks; a block inside one long
+// row gives none — (k_sell_rows) and
 // streams their chunks BH at a time, the next batch's index/value loads issued before this
 // batch's sums, so neither row boundaries nor the index loads stall the gathers; at each
 // row's end the warp folds its lanes' partials with the fixed shuffle tree and the lane
@@ -50,6 +51,7 @@ static_assert(SELL_SEG_CHUNKS / 2 < 32, "a segment's row bounds sit in one lane 
 struct SellMat {
     int64_t nrows = 0, nwin = 0, nslices = 0, slots = 0;
     int64_t nheavy = 0, nseg = 0, chunks = 0;
+    bool long_rows() const { return nheavy > 0 && chunks >= 16 * nheavy; }  // 16 or more chunks on average
     bool split = false;         // rows and windows as two launches on two streams (a large pass)
     int *ci = nullptr;          // [slots] slices
     double *v = nullptr;        // [slots]
@@ -129,20 +131,11 @@ __global__ void k_sell_chunk_counts(const int *__restrict__ rp, const int *__res
     }
 }
 
-// Per segment k (and the end, k = nseg): its first warp row, the first whose first chunk is
-// at or past k·SELL_SEG_CHUNKS (a binary search over the chunk offsets).
-__global__ void k_sell_segments(const int64_t *__restrict__ choff, int64_t nheavy, int64_t nseg,
-                                int *__restrict__ segrow) {
-    for (int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; k <= nseg; k += (int64_t)gridDim.x * blockDim.x) {
-        const int64_t c = k * SELL_SEG_CHUNKS;
-        int64_t lo = 0, hi = nheavy;  // choff[nheavy] is the total: every block start is at most it
-        while (lo < hi) {
-            const int64_t mid = (lo + hi) / 2;
-            if (choff[mid] < c) lo = mid + 1;
-            else hi = mid;
-        }
-        segrow[k] = (int)(k == nseg ? nheavy : lo);
-    }
+// Per warp row: 1 where it is the first to start in its block of SELL_SEG_CHUNKS chunks, hence
+// the first of a segment; 1 for the end, h = nheavy, too.
+__global__ void k_sell_segments(const int64_t *__restrict__ choff, int64_t nheavy, int *__restrict__ first) {
+    for (int64_t h = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; h <= nheavy; h += (int64_t)gridDim.x * blockDim.x)
+        first[h] = h == 0 || h == nheavy || choff[h] / SELL_SEG_CHUNKS != choff[h - 1] / SELL_SEG_CHUNKS;
 }
 
 // One thread per slice position: copies its row's entries to their column-major slots.
@@ -201,7 +194,6 @@ __device__ __forceinline__ void sell_rows_body(Op &op, const SellArgs &S, int64_
     double part[1] = {0.0};
     const int64_t h0 = S.segrow[seg];
     const int nr = S.segrow[seg + 1] - (int)h0;
-    if (nr == 0) return;  // a block inside one long row
     // lane k < nr: row k of the segment and its inputs; lanes 0..nr: the chunk bounds
     int row = 0;
     int64_t bound = 0;
@@ -276,11 +268,12 @@ __device__ __forceinline__ void sell_rows_body(Op &op, const SellArgs &S, int64_
     finish();
 }
 
-// The warp rows of a FUSED pass on the SELL copy: one segment per warp; MINB CTAs per SM.
+// The warp rows of a FUSED pass on the SELL copy: one segment per warp; at least MINB·NT threads
+// per SM, in CTAs of NT or less.
 template <class Op, int BH, int MINB>
 __global__ void __launch_bounds__(NT, MINB) k_sell_rows(Op op, SellArgs S) {
     if (!op.setup()) return;
-    const int64_t seg = (int64_t)blockIdx.x * (NT / 32) + (threadIdx.x >> 5);
+    const int64_t seg = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     if (seg < S.nseg) sell_rows_body<Op, BH>(op, S, seg);
 }
 
@@ -425,7 +418,6 @@ __global__ void __launch_bounds__(NT) k_sell_chk(Op op, SellArgs S, double *cont
         if (seg >= S.nseg) return;
         const int64_t h0 = S.segrow[seg];
         const int nr = S.segrow[seg + 1] - (int)h0;
-        if (nr == 0) return;
         int row = 0;
         int64_t bound = 0;
         Pre pre{};

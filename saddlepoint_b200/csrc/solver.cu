@@ -767,7 +767,9 @@ void free_sell(SellMat *S, cudaStream_t st);
 
 // Passes over at least this many nonzeros run their SELL parts on two streams; smaller
 // ones in one launch (on small LPs an iteration's time is mostly launch latency).
-constexpr int64_t SELL_SPLIT_NNZ = 4 << 20;
+// Long rows gain from the rows' own launch shape earlier (transport LP of 3.4M: an iteration
+// 52.1 µs in one launch, 48.1 in two; mixed 44.1 and 44.5).
+constexpr int64_t SELL_SPLIT_NNZ = 4 << 20, SELL_SPLIT_LONG = 1 << 20;
 
 // The SELL copy of one matrix (sell.cuh), built on the device from its CSR arrays after
 // scaling: the rows' sort keys and a stable radix sort of them (each window's rows by
@@ -838,18 +840,27 @@ int build_sell(sp_solver *s, const DevCsr &M, SellMat *S) {
     k_sell_chunk_counts<<<grid_of(s->ctx, (int64_t)nh + 1), NT, 0, st>>>(M.rp, S->heavy, nh, cnt);
     size_t b3 = 0;
     SP_CUDA_TRY(cub::DeviceScan::ExclusiveSum(nullptr, b3, cnt, S->choff, (int64_t)nh + 1, st));
-    if (b3 > btmp) {
+    // the segments' first rows, the end behind them: blocks inside one long row have none
+    int *first = nullptr, starts = 0;
+    size_t b4 = 0;
+    SP_CUDA_TRY(cub::DeviceSelect::Flagged(nullptr, b4, rows, first, S->segrow, nsel, nh + 1, st));
+    if (std::max(b3, b4) > btmp) {
         dfree(tmp, st);
         tmp = nullptr;
-        if ((rc = dmalloc(&tmp, b3))) return fail(rc);
+        if ((rc = dmalloc(&tmp, std::max(b3, b4)))) return fail(rc);
     }
     SP_CUDA_TRY(cub::DeviceScan::ExclusiveSum(tmp, b3, cnt, S->choff, (int64_t)nh + 1, st));
+    if ((rc = dmalloc((void **)&S->segrow, sizeof(int) * ((int64_t)nh + 1))) ||
+        (rc = dmalloc((void **)&first, sizeof(int) * ((int64_t)nh + 1))))
+        return fail(rc);
+    k_sell_segments<<<grid_of(s->ctx, (int64_t)nh + 1), NT, 0, st>>>(S->choff, nh, first);
+    SP_CUDA_TRY(cub::DeviceSelect::Flagged(tmp, b4, rows, first, S->segrow, nsel, nh + 1, st));
+    dfree(first, st);
     SP_CUDA_TRY(cudaMemcpyAsync(&S->chunks, S->choff + nh, sizeof(int64_t), cudaMemcpyDeviceToHost, st));
+    SP_CUDA_TRY(cudaMemcpyAsync(&starts, nsel, sizeof(int), cudaMemcpyDeviceToHost, st));
     SP_CUDA_TRY(cudaStreamSynchronize(st));
-    S->nseg = (S->chunks + SELL_SEG_CHUNKS - 1) / SELL_SEG_CHUNKS;
-    if ((rc = dmalloc((void **)&S->segrow, sizeof(int) * (S->nseg + 1)))) return fail(rc);
-    k_sell_segments<<<grid_of(s->ctx, S->nseg + 1), NT, 0, st>>>(S->choff, nh, S->nseg, S->segrow);
-    S->split = M.nnz >= SELL_SPLIT_NNZ;
+    S->nseg = nh > 0 ? starts - 1 : 0;
+    S->split = M.nnz >= (S->long_rows() ? SELL_SPLIT_LONG : SELL_SPLIT_NNZ);
     // rows too uneven for slices: more padding than the pass would save
     if (S->slots + 32 * S->chunks > SELL_MAX_SLOTS_PER_NNZ * std::max<int64_t>(M.nnz, 1024)) return fail(SP_OK);
     const int64_t hs = 32 * S->chunks;
@@ -900,8 +911,12 @@ void launch_sell_check(sp_solver *s, const SellMat &S, const DevCsr &M, cudaStre
 // FP64 (primal pass 0.276; 4 chunks at 3 CTAs/SM 0.290, 4 or 8 at the registers' natural
 // occupancy 0.288–0.293), 4 at 4 CTAs/SM in FP32 (0.255; 2 chunks 0.264); windows with 8
 // slice entries in flight at 4 CTAs/SM in both (1,024-row windows: dual pass 0.193 FP64, 0.191 FP32; 4 entries
-// 0.198, 8 at natural occupancy 0.207, 16 0.233). On the transport LP's 63-chunk rows, 4
-// chunks per batch: dual pass 0.053 ms (2 chunks 0.060, 8 0.060).
+// 0.198, 8 at natural occupancy 0.207, 16 0.233). Long rows (SellMat::long_rows), of which there
+// are few, one to a warp: 4 chunks per batch, and CTAs of 4 warps, which spread over the SMs
+// more evenly where only some rows are slow. On the transport LP's 4,000 rows of 63 chunks, half
+// of which gather with a stride, an iteration took 113.8 µs with a warp for each block, half
+// of them without a row; 102.0 without those, 95.8 with CTAs of 4 warps (2 warps 95.3; 8 chunks
+// per batch 106); mixed 99.2, 87.9, 85.1.
 template <class Op>
 void launch_sell(sp_solver *s, const SellMat &S, cudaStream_t st, const Op &op) {
     const SellArgs a = sell_args(S);
@@ -915,10 +930,10 @@ void launch_sell(sp_solver *s, const SellMat &S, cudaStream_t st, const Op &op) 
     if (rows) {
         cudaEventRecord(s->fork, st);
         cudaStreamWaitEvent(s->aux, s->fork, 0);
-        const unsigned gr = (unsigned)((S.nseg + NT / 32 - 1) / (NT / 32));
-        // rows of 16+ chunks on average (the transport LP's 63): 4 chunks per batch
-        if (sizeof(typename Op::VT) == 4 || S.chunks >= 16 * S.nheavy) k_sell_rows<Op, 4, 4><<<gr, NT, 0, s->aux>>>(op, a);
-        else k_sell_rows<Op, 2, 4><<<gr, NT, 0, s->aux>>>(op, a);
+        const int bt = S.long_rows() ? 128 : NT;
+        const unsigned gr = (unsigned)((S.nseg + bt / 32 - 1) / (bt / 32));
+        if (sizeof(typename Op::VT) == 4 || S.long_rows()) k_sell_rows<Op, 4, 4><<<gr, bt, 0, s->aux>>>(op, a);
+        else k_sell_rows<Op, 2, 4><<<gr, bt, 0, s->aux>>>(op, a);
     }
     // FP32 values: 5 CTAs per SM (0.176 ms against 0.182 at 4, with 512-row windows)
     if constexpr (sizeof(typename Op::VT) == 4) k_sell_win<Op, 8, 5><<<(unsigned)S.nwin, NT, 0, st>>>(op, a);
@@ -1257,8 +1272,8 @@ int grid_order(sp_solver *s, const DevCsr &D, const ResSrc<int> &M, const int *f
 // 2M 36.1 | 28.7, 12M 168 | 144, 16M 222 | 191; power law 60k 11.3 | 11.2, 500k 15.1 | 13.0,
 // 3M 47.0 | 40.8, 10M 128 | 107, 22M 253 | 239, 40M 446 | 434 for 100 ms more of set-up: hence
 // GRID_MAX_NNZ. Transport, whose gathers are consecutive or of a small vector, so that the
-// stream engine's wide loads count: 500k 11.3 | 10.9, 1.6M 36.9 | 26.6, 3.4M 51.9 | 52.9, 8M
-// 113 | 115 (mixed 3.4M 43.7 | 51.3): hence GRID_MAX_LONG for rows of GRID_LONG_ROW on average.
+// stream engine's wide loads count: 500k 11.3 | 10.9, 1.6M 31.3 | 26.6, 3.4M 47.7 | 52.9, 8M
+// 96 | 115 (mixed 3.4M 44.5 | 51.3): hence GRID_MAX_LONG for rows of GRID_LONG_ROW on average.
 //
 // The power iteration (ms, launches | grid): 80k 0.88 | 0.48, 200k 3.67 | 2.20, 500k 3.62 | 2.18,
 // 1M 5.35 | 3.80, 2M 5.06 | 4.48, 3M 10.3 | 10.6. From 1M on the norms' chains of additions,
