@@ -102,7 +102,7 @@ int batch_create(sp_ctx *ctx, const sp_lp *lps, int count, const sp_solver_param
                  bool tune);
 
 // Work counters of a batch: the tuned kernel's, the on-chip classes', and the instances started.
-constexpr int RES_CLASSES = 3;                      // clusters of 1, 2 and 4 CTAs
+constexpr int RES_CLASSES = 4;                      // res_class
 constexpr int BATCH_COUNTERS = 1 + RES_CLASSES + 1;
 
 int calibrate(sp_ctx *ctx, TuneTable *T) {
@@ -228,19 +228,35 @@ int tune_variants(sp_batch *b) {
 
 constexpr int RES_BATCH_SMEM = (int)STREAM_SMEM_MAX - 4096;  // dynamic shared memory, beside ResShared
 
-// The plans of the instances that run on chip, by class (clusters of 1 << class CTAs).
+// The classes, in the order in which an instance tries them: CTAs of a cluster, and the columns and
+// rows that each may have. Of a few CTAs with large parts and more with small ones the fewer
+// give the greater throughput, although an instance by itself takes longer: 192 LPs of 513-1,024
+// rows take 704 iterations with set-up in 10.8 ms with one large part each and in 10.9 with two
+// small ones, in a mix that keeps all SMs busy a fifth less; 186 of 1,025-2,000 rows in 19.1 ms
+// with two large parts and in 22.3 with four small ones. Small parts where they do: 193 of
+// 256-512 rows in 4.6 ms (large: 5.3). Four CTAs serve what two cannot split evenly.
+struct ResClass {
+    int ctas, cols, rows;
+};
+ResClass res_class(int k) {
+    static constexpr ResClass C[RES_CLASSES] = {{1, RES_SMALL_PT, RES_SMALL_PA},
+                                                {1, RES_LARGE_PT, RES_LARGE_PA},
+                                                {2, RES_LARGE_PT, RES_LARGE_PA},
+                                                {4, RES_SMALL_PT, RES_SMALL_PA}};
+    return C[k];
+}
+
+// The plans of the instances that run on chip, by class.
 struct ResBatchPlan {
     std::vector<ResBatchInst> inst;           // by instance; id = -1: not on chip
     std::vector<int> cls;
     std::vector<ResPlan> a, t;
 };
 
-// Which instances run on chip, and how: the smallest cluster whose CTAs hold the instance's
-// rows and columns (clusters cost throughput: four CTAs take a 1,900 x 3,800 LP 4.3 µs an
-// iteration, one takes a 400 x 800 LP 2.9 µs); not those with a row longer than a tile, and
-// none when another variant is forced. An instance's choice depends on it alone. Measured on
+// Which instances run on chip, and how: in the first class whose CTAs hold the instance's rows
+// and columns; not those with a row longer than a tile, and none when another variant is forced. An instance's choice depends on it alone. Measured on
 // 1,024 LPs of 50-2,000 rows, 640 iterations each with set-up (B200): 202 ms with the tuned
-// variants, 36 ms on chip.
+// variants, 30.5 ms on chip.
 ResBatchPlan plan_resident(sp_batch *b, const std::vector<int> &arp, const std::vector<int> &trp) {
     ResBatchPlan P;
     const int count = b->count;
@@ -263,17 +279,22 @@ ResBatchPlan plan_resident(sp_batch *b, const std::vector<int> &arp, const std::
             for (int r = 0; r < I.n; ++r) longest = std::max(longest, rt[r + 1] - rt[r]);
             if (longest > TILE_NNZ) continue;
             for (int k = 0; k < RES_CLASSES; ++k) {
-                const int nc = 1 << k;
-                if (I.m > nc * RES_BATCH_PA || I.n > nc * RES_BATCH_PT) continue;
+                const ResClass c = res_class(k);
+                const int nc = c.ctas;
+                if (I.m > nc * c.rows || I.n > nc * c.cols) continue;
                 ResPlan &A = P.a[i], &T = P.t[i];
                 A = ResPlan{};
                 T = ResPlan{};
                 res_plan(ra, I.m, nc, true, &A);
                 res_plan(rt, I.n, nc, true, &T);
-                if (A.most_rows > RES_BATCH_PA || T.most_rows > RES_BATCH_PT) continue;
+                if (A.most_rows > c.rows || T.most_rows > c.cols) continue;
                 auto bytes = [&](bool es) {
-                    return ResBatchPlaces(I.m, I.n, b->mixed, A.most_tasks, T.most_tasks, A.most_slots, T.most_slots, es, 8)
-                        .total;
+                    auto total = [&](auto places) { return places.total; };
+                    return c.cols == RES_LARGE_PT
+                               ? total(ResPlaces<RES_LARGE_PT, RES_LARGE_PA>(I.m, I.n, b->mixed, A.most_tasks, T.most_tasks,
+                                                                             A.most_slots, T.most_slots, es, 8))
+                               : total(ResPlaces<RES_SMALL_PT, RES_SMALL_PA>(I.m, I.n, b->mixed, A.most_tasks, T.most_tasks,
+                                                                             A.most_slots, T.most_slots, es, 8));
                 };
                 if (bytes(false) > RES_BATCH_SMEM) continue;
                 q.id = i;
@@ -301,27 +322,30 @@ ResBatchPlan plan_resident(sp_batch *b, const std::vector<int> &arp, const std::
     return P;
 }
 
-template <int NC>
+template <int NC, int PT, int PA>
 const void *res_batch_kernel(bool mixed) {
-    return mixed ? (const void *)k_batch_res<NC, true> : (const void *)k_batch_res<NC, false>;
+    return mixed ? (const void *)k_batch_res<NC, true, PT, PA> : (const void *)k_batch_res<NC, false, PT, PA>;
 }
 const void *res_batch_kernel(int cls, bool mixed) {
-    return cls == 0 ? res_batch_kernel<1>(mixed) : cls == 1 ? res_batch_kernel<2>(mixed) : res_batch_kernel<4>(mixed);
+    return cls == 0   ? res_batch_kernel<1, RES_SMALL_PT, RES_SMALL_PA>(mixed)
+           : cls == 1 ? res_batch_kernel<1, RES_LARGE_PT, RES_LARGE_PA>(mixed)
+           : cls == 2 ? res_batch_kernel<2, RES_LARGE_PT, RES_LARGE_PA>(mixed)
+                      : res_batch_kernel<4, RES_SMALL_PT, RES_SMALL_PA>(mixed);
 }
 
 // The launch of a class: its clusters, one CTA to an SM.
 int resident_config(sp_batch *b, int cls, unsigned clusters, cudaStream_t st, cudaLaunchConfig_t *cfg,
                     cudaLaunchAttribute *at) {
     *cfg = cudaLaunchConfig_t{};
-    cfg->gridDim = dim3(clusters << cls);
+    cfg->gridDim = dim3(clusters * (unsigned)res_class(cls).ctas);
     cfg->blockDim = dim3(RES_BT);
     cfg->dynamicSmemBytes = RES_BATCH_SMEM;
     cfg->stream = st;
     at->id = cudaLaunchAttributeClusterDimension;
-    at->val.clusterDim.x = 1u << cls;
+    at->val.clusterDim.x = (unsigned)res_class(cls).ctas;
     at->val.clusterDim.y = 1;
     at->val.clusterDim.z = 1;
-    if (cls) {
+    if (res_class(cls).ctas > 1) {
         cfg->attrs = at;
         cfg->numAttrs = 1;
     }
@@ -382,7 +406,7 @@ int upload_resident(sp_batch *b, const ResBatchPlan &P, const std::vector<int> &
         cudaLaunchAttribute at;
         if ((rc = resident_config(b, k, 1, st, &cfg, &at))) return rc;
         int most = 0;
-        if (k) SP_CUDA_TRY(cudaOccupancyMaxActiveClusters(&most, res_batch_kernel(k, b->mixed), &cfg));
+        if (res_class(k).ctas > 1) SP_CUDA_TRY(cudaOccupancyMaxActiveClusters(&most, res_batch_kernel(k, b->mixed), &cfg));
         else most = b->ctx->sms;
         b->res_clusters[k] = std::max(1, std::min(c.count, most));
         c.counter = b->args.counter + 1 + k;

@@ -13,9 +13,9 @@
 
 namespace sp {
 
-constexpr int RES_BATCH_PT = 1024, RES_BATCH_PA = 512;  // columns and rows of a CTA
-constexpr int RES_BATCH_MAX = 4;                        // CTAs of an instance at most
-using ResBatchPlaces = ResPlaces<RES_BATCH_PT, RES_BATCH_PA>;
+constexpr int RES_BATCH_MAX = 4;  // CTAs of an instance at most
+// Columns and rows of a CTA: classes of small and of large parts.
+constexpr int RES_SMALL_PT = 1024, RES_SMALL_PA = 512, RES_LARGE_PT = 2048, RES_LARGE_PA = 1024;
 
 // The plan of one instance: offsets into the plan arenas (BatchRes) and sizes.
 struct ResBatchInst {
@@ -236,7 +236,7 @@ __device__ __noinline__ void res_scale(ResShared<uint16_t> &sh, const BatchArgs 
 // bound norm and cost norm of the scaled problem, then of the original.
 __device__ __noinline__ void res_norms(const double *olc, const double *ouc, const double *oc, const double *rs,
                                        const double *cs, int m, int n, double (&out)[4]) {
-    constexpr int CH = RES_BATCH_PT;  // terms of a chunk: X, XA, C and LV hold one norm's each
+    constexpr int CH = RES_SMALL_PT;  // terms of a chunk: X, XA, C and LV hold one norm's each
     double *term = &dsm_at<double>(0);
     double s = -0.0;
     for (int base = 0; base < max(m, n); base += CH) {
@@ -293,18 +293,19 @@ struct ResBatchShared {
     float next;     // the instance's number (below 2^24), by cluster_store
 };
 
-__device__ __forceinline__ ResBatchPlaces res_batch_places(const ResBatchInst &I, int m, int n, bool mixed, bool es) {
-    return ResBatchPlaces(m, n, mixed, I.mostA[2], I.mostT[2], I.mostA[1], I.mostT[1], es, 8);
+template <int PT, int PA>
+__device__ __forceinline__ ResPlaces<PT, PA> res_batch_places(const ResBatchInst &I, int m, int n, bool mixed, bool es) {
+    return ResPlaces<PT, PA>(m, n, mixed, I.mostA[2], I.mostT[2], I.mostA[1], I.mostT[1], es, 8);
 }
 
 // Everything before the PDHG epochs: the entries, the scaling, the norms, ‖A'‖₂ and the start.
-template <int NC, bool MIXED, bool ES>
+template <int NC, bool MIXED, bool ES, int PT, int PA>
 __device__ __noinline__ void res_batch_setup(const BatchArgs &A, const BatchRes &B, const ResBatchInst &I,
                                              unsigned char *scratch, ResBatchShared &bsh) {
     ResShared<uint16_t> &s = bsh.s;
     const BatchInst &D = A.inst[I.id];
     const int m = D.m, n = D.n, c = res_rank<NC>();
-    const ResBatchPlaces L = res_batch_places(I, m, n, MIXED, ES);
+    const auto L = res_batch_places<PT, PA>(I, m, n, MIXED, ES);
     const ResScratch W(I.sA[NC], I.sT[NC], m, n, D.nta, D.ntt, MIXED);
     auto src = [&](bool a) {
         ResSrc<uint16_t> q{};
@@ -486,7 +487,7 @@ __device__ __noinline__ void res_batch_finish(const BatchArgs &A, const ResBatch
 }
 
 // One class of instances: clusters of NC CTAs take them from the class's counter.
-template <int NC, bool MIXED>
+template <int NC, bool MIXED, int PT, int PA>
 __global__ void __launch_bounds__(RES_BT, 1)
     k_batch_res(const __grid_constant__ BatchArgs A, const __grid_constant__ BatchRes B,
                 const __grid_constant__ ResBatchClass K) {
@@ -505,10 +506,10 @@ __global__ void __launch_bounds__(RES_BT, 1)
         const ResBatchInst &I = K.inst[slot];
         auto solve = [&](auto in_shared) {
             constexpr bool ES = decltype(in_shared)::value;
-            res_batch_setup<NC, MIXED, ES>(A, B, I, scratch, b);
-            const ResBatchPlaces L = res_batch_places(I, b.s.R.A.rows, b.s.R.T.rows, MIXED, ES);
+            res_batch_setup<NC, MIXED, ES, PT, PA>(A, B, I, scratch, b);
+            const auto L = res_batch_places<PT, PA>(I, b.s.R.A.rows, b.s.R.T.rows, MIXED, ES);
             if constexpr (MIXED) {
-                res_epochs<NC, true, ES>(b.s, L, stop);
+                res_epochs<NC, true, ES, ES>(b.s, L, stop);
                 res_sync<NC>();
                 if (ES && !b.s.st.done) {
                     res_load_entries<double>(b.s.R.A, b.s.R.A.v, L.valA, L.atA, L.xbar);
@@ -516,7 +517,7 @@ __global__ void __launch_bounds__(RES_BT, 1)
                     __syncthreads();
                 }
             }
-            res_epochs<NC, false, ES>(b.s, L, stop);
+            res_epochs<NC, false, ES, ES>(b.s, L, stop);
             res_sync<NC>();
         };
         if (I.es) solve(std::true_type{});

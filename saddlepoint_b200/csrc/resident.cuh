@@ -886,8 +886,11 @@ struct ResPeers {
     }
 };
 
-// `its` FUSED iterations from Halpern counter k0.
-template <int NC, bool LO, bool ES, int PT, int PA>
+// `its` FUSED iterations from Halpern counter k0. HEADS: each pass's first head stays in registers.
+// With entries in global memory that suits a kernel with room for it (a 3,500 x 7,000 LP in
+// the solver's: 5.7 µs an iteration, 6.1 without), not the batch's, whose shorter paths then
+// spill (its 1,024 LPs of 50-2,000 rows: 32.0 ms, 30.5 without).
+template <int NC, bool LO, bool ES, bool HEADS, int PT, int PA>
 __device__ __forceinline__ void res_iterate(ResShared<uint16_t> &sh, const ResPlaces<PT, PA> &L, unsigned long long k0,
                                             unsigned long long its) {
     using VT = typename std::conditional<LO, float, double>::type;
@@ -912,8 +915,8 @@ __device__ __forceinline__ void res_iterate(ResShared<uint16_t> &sh, const ResPl
     const int t0 = (&dsm_at<int>(L.wtT))[warp], t1 = (&dsm_at<int>(L.wtT))[warp + 1];
     const int a0 = (&dsm_at<int>(L.wtA))[warp], a1 = (&dsm_at<int>(L.wtA))[warp + 1];
     ResHead<VT> hT, hA;
-    if (t0 < t1) hT.load(ET, (&dsm_at<ResTask>(L.tasksT))[t0], gy + (int)sizeof(VT) * sh.R.A.rows);
-    if (a0 < a1) hA.load(EA, (&dsm_at<ResTask>(L.tasksA))[a0], gx + (int)sizeof(VT) * sh.R.T.rows);
+    if (HEADS && t0 < t1) hT.load(ET, (&dsm_at<ResTask>(L.tasksT))[t0], gy + (int)sizeof(VT) * sh.R.A.rows);
+    if (HEADS && a0 < a1) hA.load(EA, (&dsm_at<ResTask>(L.tasksA))[a0], gx + (int)sizeof(VT) * sh.R.T.rows);
     double w = 0.0;
     // A task's rows: PrimalPass and DualPass with MODE 0 (solver_kernels.cuh) on positions.
     auto primal = [&](const ResTask t, const ResHead<VT> *head) {
@@ -955,11 +958,11 @@ __device__ __forceinline__ void res_iterate(ResShared<uint16_t> &sh, const ResPl
 #pragma unroll 1
         for (int i = 0; i < cnt; ++i) {
             w = sh.wtab[i];
-            if (t0 < t1) primal((&dsm_at<ResTask>(L.tasksT))[t0], &hT);
+            if (t0 < t1) primal((&dsm_at<ResTask>(L.tasksT))[t0], HEADS ? &hT : nullptr);
 #pragma unroll 1
             for (int ti = t0 + 1; ti < t1; ++ti) primal((&dsm_at<ResTask>(L.tasksT))[ti], nullptr);
             res_sync<NC>();
-            if (a0 < a1) dual((&dsm_at<ResTask>(L.tasksA))[a0], &hA);
+            if (a0 < a1) dual((&dsm_at<ResTask>(L.tasksA))[a0], HEADS ? &hA : nullptr);
 #pragma unroll 1
             for (int ti = a0 + 1; ti < a1; ++ti) dual((&dsm_at<ResTask>(L.tasksA))[ti], nullptr);
             res_sync<NC>();
@@ -1085,7 +1088,7 @@ __device__ __noinline__ void res_check(ResShared<IX> &sh, unsigned long long E, 
 // Epochs of check_every iterations (the last one cut at max_iterations), each ended by its
 // check, until the state is done, its total has reached sh.until, or (mixed form) the other
 // precision is due: LO runs the FP32 phase.
-template <int NC, bool LO, bool ES, int PT, int PA, class Stop>
+template <int NC, bool LO, bool ES, bool HEADS, int PT, int PA, class Stop>
 __device__ __forceinline__ void res_epochs(ResShared<uint16_t> &sh, const ResPlaces<PT, PA> &L, Stop stop) {
     while (!sh.st.done && sh.st.total < sh.until && LO == (sh.mixed && !sh.st.fp64)) {
         unsigned long long E = sh.prm.max_iterations > sh.st.total ? sh.prm.max_iterations - sh.st.total : 1;
@@ -1095,7 +1098,7 @@ __device__ __forceinline__ void res_epochs(ResShared<uint16_t> &sh, const ResPla
             res_first<NC, LO>(sh);
             if (sh.st.done) break;
         }
-        res_iterate<NC, LO, ES>(sh, L, sh.st.k + first, E - 1 - first);
+        res_iterate<NC, LO, ES, HEADS>(sh, L, sh.st.k + first, E - 1 - first);
         res_check<NC, LO>(sh, E, stop);
     }
 }
@@ -1267,7 +1270,7 @@ __global__ void __launch_bounds__(RES_BT, 1) k_res_epochs(const __grid_constant_
         if (LO) S.y32[k] = (float)v;
     }
     res_sync<NC>();
-    res_epochs<NC, LO, ES>(s, L, ResNoStop{});
+    res_epochs<NC, LO, ES, true>(s, L, ResNoStop{});
     res_sync<NC>();
     for (int k = R.T.p0 + threadIdx.x; k < R.T.p1; k += RES_BT) {
         const int j = R.T.perm[k];
