@@ -21,12 +21,13 @@ namespace sp {
 
 // The grid's barrier: counts arrivals in global memory and waits for them. The launch is
 // cooperative, so every CTA is running. What was written to global memory before it is visible
-// after it. The wait is bounded (GRID_WAIT_NS, or another CTA's giving up); a CTA that gives
+// after it. The wait is bounded (GRID_WAIT_NS; GRID_START_NS at a kernel's first barrier, which
+// waits until kernels of other streams, a batch's say, have left all SMs; or another CTA's giving up); a CTA that gives
 // up marks itself and all later barriers let it through, so that the kernel ends, and the
 // solve is reported as failed. 1.2 µs for 148 CTAs (B200); counting in two levels took 1.7.
 // A long wait is one for SMs that another kernel holds; it polls at intervals, since 144 CTAs
 // polling without pause slowed that kernel down eightfold (the set-up's norms: 6 ms to 46).
-constexpr unsigned long long GRID_WAIT_NS = 10000000000ull, GRID_SPIN_NS = 100000ull;
+constexpr unsigned long long GRID_START_NS = 600000000000ull, GRID_WAIT_NS = 10000000000ull, GRID_SPIN_NS = 100000ull;
 struct GridBar {
     unsigned count, abort;
 };
@@ -42,7 +43,7 @@ __device__ __forceinline__ unsigned ld_acquire(const unsigned *p) {
     return v;
 }
 
-__device__ __forceinline__ void grid_sync(GridState &g) {  // g: a shared variable
+__device__ __forceinline__ void grid_sync(GridState &g, unsigned long long limit = GRID_WAIT_NS) {  // g: a shared variable
     __syncthreads();
     if (threadIdx.x == 0 && !g.dead) {
         const unsigned target = g.passed + gridDim.x;
@@ -51,7 +52,7 @@ __device__ __forceinline__ void grid_sync(GridState &g) {  // g: a shared variab
             const unsigned long long t0 = global_ns();
             while (ld_acquire(&g.bar->count) < target) {
                 const unsigned long long waited = global_ns() - t0;
-                if (ld_acquire(&g.bar->abort) || waited > GRID_WAIT_NS) {
+                if (ld_acquire(&g.bar->abort) || waited > limit) {
                     atomicExch(&g.bar->abort, 1u);
                     g.dead = 1;
                     break;
@@ -402,7 +403,7 @@ __global__ void __launch_bounds__(RES_BT, 1) k_grid_mid(const __grid_constant__ 
         a.y[k] = yn;
         if constexpr (LO) gy[k] = (float)yn;
     };
-    grid_sync(sh.grid);
+    grid_sync(sh.grid, GRID_START_NS);
     const unsigned long long k0 = a.g.st->k;
 #pragma unroll 1
     for (int i = 1; i < E - 1 && !sh.grid.dead; ++i) {
@@ -495,7 +496,7 @@ __global__ void __launch_bounds__(RES_BT, 1) k_grid_power(const __grid_constant_
     double scale = 1.0 / sqrt(s[0]), lambda = 0.0;
     int iters = 0, error = ERR_NONE;
     bool done = false;
-    grid_sync(sh.grid);
+    grid_sync(sh.grid, GRID_START_NS);
     while (!done && !sh.grid.dead) {
         grid_rows(EA, L.tasksA, a0, a1, [&](double x, double g) { return x * (g * scale); },
                   [&](int ty, int tz, double q) {

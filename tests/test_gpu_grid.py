@@ -124,6 +124,31 @@ def test_grid_solves_beside_each_other(gpu_backend):
         assert_identical(a, b)
 
 
+def test_grid_solve_beside_a_batch(gpu_backend):
+    """The grid waits for the SMs that a batch on another stream holds; both as when alone."""
+    lp = sp().generate_random_lp(40, 20000, 40000, (4, 6))
+    p = params(640)
+    alone = sp().solve(lp, p, gpu_backend)
+    lps = [sp().generate_random_lp(50 + k, 30 + 3 * k, 60 + 6 * k, (3, 8)) for k in range(300)]
+    b = sp().BatchSolver(lps, params(3000), gpu_backend)
+    want = [(r.objective, r.iterations) for r in b.solve()[0]]
+    got = []
+
+    def work():
+        be = sp().CudaBackend(0)
+        for _ in range(6):
+            got.append(sp().solve(lp, p, be))
+
+    t = threading.Thread(target=work)
+    t.start()
+    for _ in range(3):
+        assert [(r.objective, r.iterations) for r in b.solve()[0]] == want
+    t.join()
+    assert len(got) == 6
+    for g in got:
+        assert_identical(alone, g)
+
+
 def test_grid_nonfinite_iterates_are_a_numerical_error(gpu_backend):
     """Costs near the largest number overflow the first residuals: the same error as on tiles."""
     lp = sp().generate_random_lp(23, 3000, 6000, (3, 5))
