@@ -1326,6 +1326,14 @@ struct GridPlan {
     }
 };
 
+void release_grid(sp_solver *s, cudaStream_t st) {
+    for (void **p : {&s->res_mem, s->grid_slots, s->grid_slots + 1, s->grid_slots + 2, s->grid_slots + 3, s->grid_slots + 4,
+                     s->grid_slots + 5}) {
+        dfree(*p, st);
+        *p = nullptr;
+    }
+}
+
 // Sets the grid engine up from its plan.
 int grid_build(sp_solver *s, GridPlan &plan_of) {
     if (s->res_ctas || !plan_of.join()) return SP_OK;
@@ -1371,7 +1379,9 @@ int grid_build(sp_solver *s, GridPlan &plan_of) {
         SP_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, (const void *)l->f, RES_BT, (size_t)l->smem));
         if ((int64_t)per_sm * s->ctx->sms < ctas) return SP_OK;
     }
-    // one allocation: the plans, the slots and the position-space vectors
+    // the plans and the position-space vectors in one allocation, the slots in one per array: where
+    // the pool has to grow, smaller blocks are had sooner (a process's first solver, mixed, of 10M
+    // nonzeros 71 ms, 98 with one block of 350 MB; of 2M 26 and 39; on launches 77 and 25)
     size_t bytes = 0;
     auto room = [&](size_t b) {
         const size_t at = bytes;
@@ -1385,7 +1395,7 @@ int grid_build(sp_solver *s, GridPlan &plan_of) {
         return at;
     };
     struct Off {
-        size_t perm, inv, tasks, first, wt, p0, s0, ci, v, v32;
+        size_t perm, inv, tasks, first, wt, p0, s0;
     } oa{}, ot{};
     auto plan = [&](const ResCuts &P, const DevCsr &M, Off *o) {
         o->perm = room(sizeof(int) * (size_t)M.nrows);
@@ -1395,9 +1405,6 @@ int grid_build(sp_solver *s, GridPlan &plan_of) {
         o->wt = vec(P.wt);
         o->p0 = vec(P.p0);
         o->s0 = vec(P.s0);
-        o->ci = room(sizeof(int) * (size_t)P.slots);
-        o->v = room(sizeof(double) * (size_t)P.slots);
-        o->v32 = s->mixed ? room(sizeof(float) * (size_t)P.slots) : 0;
     };
     plan(PA, s->A, &oa);
     plan(PT, s->AT, &ot);
@@ -1407,24 +1414,30 @@ int grid_build(sp_solver *s, GridPlan &plan_of) {
     const size_t contrib = room(8 * N), bar = room(sizeof(GridBar));
     cudaStream_t st = s->ctx->stream;
     int rc;
-    if (dmalloc(&s->res_mem, bytes)) {  // no room for it: the launched engines need none
+    bool room_for = !dmalloc(&s->res_mem, bytes);
+    for (int q = 0; q < 6 && room_for; ++q) {  // A's positions, values and FP32 values, then A'ᵀ's
+        const size_t slots = (size_t)(q < 3 ? PA : PT).slots, width = q % 3 == 1 ? 8 : 4;
+        if (q % 3 < 2 || s->mixed) room_for = !dmalloc(&s->grid_slots[q], width * slots);
+    }
+    if (!room_for) {  // the launched engines need none
+        release_grid(s, st);
         s->ctx->last_error.clear();
         return SP_OK;
     }
     unsigned char *d = (unsigned char *)s->res_mem;
     for (const auto &u : ups) SP_CUDA_TRY(cudaMemcpyAsync(d + u.first, u.second.first, u.second.second, cudaMemcpyHostToDevice, st));
-    auto place = [&](ResSrc<int> &q, const Off &o) {
+    auto place = [&](ResSrc<int> &q, const Off &o, void *const *slots) {
         q.tasks = (const ResTask *)(d + o.tasks);
         q.wt = (const int *)(d + o.wt);
         q.p0 = (const int *)(d + o.p0);
         q.s0 = (const int *)(d + o.s0);
         q.perm = (const int *)(d + o.perm);
-        q.ci = (int *)(d + o.ci);
-        q.v = (double *)(d + o.v);
-        q.v32 = s->mixed ? (float *)(d + o.v32) : nullptr;
+        q.ci = (int *)slots[0];
+        q.v = (double *)slots[1];
+        q.v32 = (float *)slots[2];
     };
-    place(a.A, oa);
-    place(a.T, ot);
+    place(a.A, oa, s->grid_slots);
+    place(a.T, ot, s->grid_slots + 3);
     double *v = (double *)(d + inputs);
     for (double **q : {&a.x, &a.c, &a.lv, &a.uv, &a.xa}) {
         *q = v;
@@ -1677,7 +1690,7 @@ void solver_release(sp_solver *s) {
         cudaEventDestroy(s->join);
     }
     cudaStream_t fst = s->ctx->stream;
-    dfree(s->res_mem, fst);
+    release_grid(s, fst);
     free_csr(&s->A, fst);
     free_csr(&s->AT, fst);
     free_sell(&s->sellA, fst);

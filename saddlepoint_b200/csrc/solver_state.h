@@ -44,8 +44,10 @@ struct sp_solver {
     sp::ResArgs res{};
     sp::ResLaunch res_epochs[2], res_power;  // epochs in FP64 and of the FP32 phase
     void *res_mem = nullptr;
-    // a mid-sized LP's engine over the whole grid (grid.cuh; 0 CTAs: not used), its memory in res_mem
+    // a mid-sized LP's engine over the whole grid (grid.cuh; 0 CTAs: not used), its memory in
+    // res_mem and, the slots, in grid_slots
     int grid_ctas = 0;
+    void *grid_slots[6] = {};
     sp::GridArgs grid{};
     sp::GridLaunch grid_mid[2], grid_power;  // an epoch's iterations in FP64 and in the FP32 phase
     double *contrib = nullptr;   // [NP_D][m] row contributions of the check's dual pass on the SELL copy
