@@ -233,8 +233,9 @@ double sp_solver_bytes_per_iteration(sp_solver *s);
 /* Which engine runs each fused pass of the solver (chosen at creation from the
  * problem's size, or SP_PASS_ENGINE): out[0] primal FP64, out[1] primal FP32,
  * out[2] dual FP64, out[3] dual FP32 (the FP32 entries apply to the mixed form). A small
- * LP's iterations run on chip, several epochs to a launch; the engines named here then run
- * its passes only where sp_solver_set_timing has them launched one by one. */
+ * LP's iterations run on chip, several epochs to a launch, a mid-sized one's in one launch
+ * between an epoch's first and its check; the engines named here then run its other passes,
+ * and all of them where sp_solver_set_timing has them launched one by one. */
 enum { SP_ENGINE_TILES = 0, SP_ENGINE_STREAM = 1, SP_ENGINE_SELL = 2 };
 int sp_solver_engines(sp_solver *s, int32_t out[4]);
 /* The floor a pass's random gathers set: the average time of a kernel that does only
