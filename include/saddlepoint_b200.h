@@ -282,6 +282,10 @@ int sp_batch_create(sp_ctx *ctx, const sp_lp *lps, int count, const sp_solver_pa
 int sp_batch_solve(sp_batch *b, sp_batch_result *results, double *elapsed_s);
 /* x/y of instance i in the original space. */
 int sp_batch_download(sp_batch *b, int i, double *x, double *y);
+/* Where instance i runs: out[0] the CTAs of its cluster (0: not on chip, but on the kernel
+ * of the tuned variants), out[1] the columns that each CTA may have, out[2] whether the
+ * matrix entries lie in shared memory. */
+int sp_batch_engine(sp_batch *b, int i, int32_t out[3]);
 void sp_batch_free(sp_batch *b);
 
 /* ========================================================================

@@ -161,6 +161,7 @@ SIGNATURES = [
     ("sp_batch_create", cint, [VP, C.POINTER(Lp), cint, C.POINTER(Params), C.POINTER(VP)]),
     ("sp_batch_solve", cint, [VP, C.POINTER(BatchResult), PD]),
     ("sp_batch_download", cint, [VP, cint, PD, PD]),
+    ("sp_batch_engine", cint, [VP, cint, PI32]),
     ("sp_batch_free", None, [VP]),
     ("sp_server_create", cint, [VP, C.POINTER(ServerConfig), C.POINTER(Params), C.POINTER(VP)]),
     ("sp_server_submit", cint, [VP, C.POINTER(Lp), PI64]),

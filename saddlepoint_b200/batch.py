@@ -88,6 +88,13 @@ class BatchSolver:
         self.backend._check(self.lib.sp_batch_download(self.h, i, x.ctypes.data_as(L.PD), y.ctypes.data_as(L.PD)))
         return x, y
 
+    def engine(self, i: int):
+        """(CTAs, columns a CTA may have, entries in shared memory) of instance i on chip; None
+        where the kernel of the tuned variants runs it."""
+        out = (C.c_int32 * 3)()
+        self.backend._check(self.lib.sp_batch_engine(self.h, i, out))
+        return (out[0], out[1], bool(out[2])) if out[0] else None
+
 
 @dataclass
 class ServerResult:

@@ -30,7 +30,8 @@ struct sp_batch {
     std::vector<void *> bufs;
     cudaGraphExec_t graph = nullptr;
     int grid = 0;
-    int res_clusters[3] = {};  // clusters of each on-chip class
+    int res_clusters[sp::RES_CLASSES] = {};  // clusters of each on-chip class
+    std::vector<sp::BatchChip> chip;         // by instance
     sp::BatchInst *d_inst = nullptr;
     int *d_counter = nullptr;
     double *av0 = nullptr, *tv0 = nullptr;  // the original values (the kernel scales in place)
@@ -102,7 +103,6 @@ int batch_create(sp_ctx *ctx, const sp_lp *lps, int count, const sp_solver_param
                  bool tune);
 
 // Work counters of a batch: the tuned kernel's, the on-chip classes', and the instances started.
-constexpr int RES_CLASSES = 4;                      // res_class
 constexpr int BATCH_COUNTERS = 1 + RES_CLASSES + 1;
 
 int calibrate(sp_ctx *ctx, TuneTable *T) {
@@ -318,7 +318,11 @@ ResBatchPlan plan_resident(sp_batch *b, const std::vector<int> &arp, const std::
     for (int t = 0; t < nt; ++t) th.emplace_back(run, (int)((int64_t)count * t / nt), (int)((int64_t)count * (t + 1) / nt));
     for (auto &t : th) t.join();
     for (int i = 0; i < count; ++i)
-        if (P.inst[i].id >= 0) b->inst[i].variant = VARIANT_RES;
+        if (P.inst[i].id >= 0) {
+            const ResClass c = res_class(P.cls[i]);
+            b->inst[i].variant = VARIANT_RES;
+            b->chip[i] = BatchChip{c.ctas, c.cols, P.inst[i].es};
+        }
     return P;
 }
 
@@ -615,6 +619,7 @@ int batch_create(sp_ctx *ctx, const sp_lp *lps, int count, const sp_solver_param
     };
     // offsets
     b->inst.resize(count);
+    b->chip.resize(count);
     int64_t rpa = 0, rpt = 0, nz = 0, mo = 0, no = 0;
     for (int i = 0; i < count; ++i) {
         const sp_lp &L = lps[i];
@@ -958,5 +963,14 @@ extern "C" int sp_batch_download(sp_batch *b, int i, double *x, double *y) {
     const int64_t nx = E.no + E.n - F.no;
     if (x && I.n) memcpy(x, b->dl + (I.no - F.no), sizeof(double) * I.n);
     if (y && I.m) memcpy(y, b->dl + nx + (I.mo - F.mo), sizeof(double) * I.m);
+    return SP_OK;
+}
+
+extern "C" int sp_batch_engine(sp_batch *b, int i, int32_t out[3]) {
+    if (!b || !out || i < 0 || i >= b->count) return SP_ERR_INVALID;
+    const BatchChip &c = b->chip[i];
+    out[0] = c.ctas;
+    out[1] = c.cols;
+    out[2] = c.entries;
     return SP_OK;
 }

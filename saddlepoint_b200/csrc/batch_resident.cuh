@@ -14,6 +14,7 @@
 namespace sp {
 
 constexpr int RES_BATCH_MAX = 4;  // CTAs of an instance at most
+constexpr int RES_CLASSES = 4;    // the classes of instances (res_class, batch.cu)
 // Columns and rows of a CTA: classes of small and of large parts.
 constexpr int RES_SMALL_PT = 1024, RES_SMALL_PA = 512, RES_LARGE_PT = 2048, RES_LARGE_PA = 1024;
 
@@ -25,6 +26,11 @@ struct ResBatchInst {
     int heavyA, heavyT;
     int mostA[3], mostT[3];         // rows, slots, tasks of one CTA
     int pA[RES_BATCH_MAX + 1], sA[RES_BATCH_MAX + 1], pT[RES_BATCH_MAX + 1], sT[RES_BATCH_MAX + 1];
+};
+
+// Where an instance runs on chip, for sp_batch_engine (0 CTAs: not there).
+struct BatchChip {
+    int ctas = 0, cols = 0, entries = 0;
 };
 
 // The instances of one class (cluster size) and what their kernel needs.
