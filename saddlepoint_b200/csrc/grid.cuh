@@ -27,13 +27,21 @@ namespace sp {
 // solve is reported as failed. 1.2 µs for 148 CTAs (B200); counting in two levels took 1.7.
 // A long wait is one for SMs that another kernel holds; it polls at intervals, since 144 CTAs
 // polling without pause slowed that kernel down eightfold (the set-up's norms: 6 ms to 46).
+// The count wraps (148 arrivals twice an iteration: after 14.5M iterations of a launch), so
+// counts are compared by their difference, which is at most one barrier's arrivals; it starts
+// one below the wrap, so that every launch passes it.
 constexpr unsigned long long GRID_START_NS = 600000000000ull, GRID_WAIT_NS = 10000000000ull, GRID_SPIN_NS = 100000ull;
 struct GridBar {
-    unsigned count, abort;
+    unsigned count, alive;  // alive: 0 once a wait has given up
 };
+constexpr unsigned GRID_COUNT0 = ~0u;  // both words at a launch's start (one fill)
+__host__ __device__ constexpr bool grid_before(unsigned count, unsigned target) { return (int)(count - target) < 0; }
+static_assert(grid_before(GRID_COUNT0, GRID_COUNT0 + 148u) && grid_before(147u, 148u) && !grid_before(148u, 148u) &&
+                  !grid_before(3u, GRID_COUNT0) && grid_before(0xfffffff0u, 16u),
+              "counts on both sides of the wrap");
 struct GridState {
     GridBar *bar;
-    unsigned passed;  // arrivals of the barriers so far
+    unsigned passed;  // the count after the barriers so far
     int dead;         // a wait gave up
 };
 
@@ -48,12 +56,12 @@ __device__ __forceinline__ void grid_sync(GridState &g, unsigned long long limit
     if (threadIdx.x == 0 && !g.dead) {
         const unsigned target = g.passed + gridDim.x;
         asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(&g.bar->count) : "memory");
-        if (ld_acquire(&g.bar->count) < target) {
+        if (grid_before(ld_acquire(&g.bar->count), target)) {
             const unsigned long long t0 = global_ns();
-            while (ld_acquire(&g.bar->count) < target) {
+            while (grid_before(ld_acquire(&g.bar->count), target)) {
                 const unsigned long long waited = global_ns() - t0;
-                if (ld_acquire(&g.bar->abort) || waited > limit) {
-                    atomicExch(&g.bar->abort, 1u);
+                if (!ld_acquire(&g.bar->alive) || waited > limit) {
+                    atomicExch(&g.bar->alive, 0u);
                     g.dead = 1;
                     break;
                 }
@@ -103,7 +111,7 @@ struct GridArgs {
     double *y, *xbar;               // ... the gathered vectors; GRID_ONES 1.0 behind each
     float *y32, *xbar32;
     double *contrib, *ppart;        // the power iteration's
-    GridBar *bar;                   // zeroed before each launch
+    GridBar *bar;                   // all ones before each launch
     int mixed;
 };
 
@@ -124,7 +132,7 @@ template <bool VS, bool ES, int PT, int PA>
 __device__ inline void grid_open(GridShared &sh, const GridPlaces<VS, ES, PT, PA> &L, const GridArgs &a) {
     const int c = (int)blockIdx.x;
     if (threadIdx.x == 0) {
-        sh.grid = GridState{a.bar, 0, 0};
+        sh.grid = GridState{a.bar, GRID_COUNT0, 0};
         sh.A = res_side(a.A, c, L.tasksA, L.wtA);
         sh.T = res_side(a.T, c, L.tasksT, L.wtT);
     }
@@ -297,7 +305,7 @@ __device__ __forceinline__ void grid_rows(const GridEntries<VT, ES> &E, int task
 // vectors' initial state is read from the row-ordered vectors and left there again; x, c, lv, uv
 // and the like lie over positions: c, lv, uv, lc, uc since the solver was made.
 template <bool LO, bool VS, bool ES, int PT, int PA>
-__global__ void __launch_bounds__(RES_BT, 1) k_grid_mid(const __grid_constant__ GridArgs a, int E) {
+__global__ void __launch_bounds__(RES_BT, 1) k_grid_mid(const __grid_constant__ GridArgs a, long long E) {
     using VT = typename std::conditional<LO, float, double>::type;
     using P = GridPlaces<VS, ES, PT, PA>;
     __shared__ GridShared sh;
@@ -406,10 +414,10 @@ __global__ void __launch_bounds__(RES_BT, 1) k_grid_mid(const __grid_constant__ 
     grid_sync(sh.grid, GRID_START_NS);
     const unsigned long long k0 = a.g.st->k;
 #pragma unroll 1
-    for (int i = 1; i < E - 1 && !sh.grid.dead; ++i) {
+    for (unsigned long long i = 1; i + 1 < (unsigned long long)E && !sh.grid.dead; ++i) {
         if (i == 1 || i % RES_WTAB == 0) {  // every reader of the last weights is past a barrier
             if (threadIdx.x < RES_WTAB) {
-                const unsigned long long k = k0 + (unsigned long long)(i / RES_WTAB * RES_WTAB) + threadIdx.x;
+                const unsigned long long k = k0 + i / RES_WTAB * RES_WTAB + threadIdx.x;
                 sh.wtab[threadIdx.x] = (double)(k + 1) / (double)(k + 2);
             }
             __syncthreads();
@@ -466,7 +474,7 @@ static __global__ void k_grid_inputs(GridArgs a) {
 
 // The solver's power iteration (res_power's: the same start, sums and stopping rule).
 template <bool ES>
-__global__ void __launch_bounds__(RES_BT, 1) k_grid_power(const __grid_constant__ GridArgs a, int max_iters) {
+__global__ void __launch_bounds__(RES_BT, 1) k_grid_power(const __grid_constant__ GridArgs a, long long max_iters) {
     __shared__ GridShared sh;
     const auto L = grid_places<false, ES, 0, 0>(a, false);
     grid_open(sh, L, a);

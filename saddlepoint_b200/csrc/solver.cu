@@ -32,7 +32,7 @@ namespace sp {
 struct CtrlArgs {
     const double *partP, *partD, *partT, *partP0, *partD0;
     int nP, nD;  // tiles of A'ᵀ and of A'
-    int E;       // iterations in this epoch
+    long long E; // iterations in this epoch
     sp_check_record *trace;
     long long trace_cap;
 };
@@ -656,7 +656,7 @@ SolverPtrs ptrs_of(sp_solver *s) {
 }
 
 template <bool LO, int MODE>
-PrimalPass<LO, MODE> mkP(const SolverPtrs &p, int i, int role) {
+PrimalPass<LO, MODE> mkP(const SolverPtrs &p, long long i, int role) {
     PrimalPass<LO, MODE> o{};
     o.rp = p.t_rp;
     o.ci = p.t_ci;
@@ -670,7 +670,7 @@ PrimalPass<LO, MODE> mkP(const SolverPtrs &p, int i, int role) {
     return o;
 }
 template <bool LO, int MODE>
-DualPass<LO, MODE> mkD(const SolverPtrs &p, int i, int role) {
+DualPass<LO, MODE> mkD(const SolverPtrs &p, long long i, int role) {
     DualPass<LO, MODE> o{};
     o.rp = p.a_rp;
     o.ci = p.a_ci;
@@ -1206,9 +1206,9 @@ void split_ranges(int64_t len, const F &body) {
 constexpr int GRID_PT = 1024, GRID_PA = 512;     // columns and rows of a CTA with entries in shared memory
 constexpr int GRID_PT2 = 2560, GRID_PA2 = 1280;  // ... without
 
-int grid_launch(const sp_solver *s, const GridLaunch &l, int n) {
+int grid_launch(const sp_solver *s, const GridLaunch &l, long long n) {
     cudaStream_t st = s->ctx->stream;
-    SP_CUDA_TRY(cudaMemsetAsync(s->grid.bar, 0, sizeof(GridBar), st));
+    SP_CUDA_TRY(cudaMemsetAsync(s->grid.bar, GRID_COUNT0 & 0xff, sizeof(GridBar), st));
     void *args[] = {(void *)&s->grid, (void *)&n};
     SP_CUDA_TRY(cudaLaunchCooperativeKernel((const void *)l.f, dim3((unsigned)s->grid_ctas), dim3(RES_BT), args,
                                             (size_t)l.smem, st));
@@ -1474,7 +1474,7 @@ int grid_build(sp_solver *s, GridPlan &plan_of) {
 // Launches the primal pass of iteration i with the given role. MID iterations go
 // through the stream engine when it is on (in the mixed form one launch per
 // precision; the one that does not match the device state returns at once).
-void launch_P(sp_solver *s, int i, int role, cudaStream_t st) {
+void launch_P(sp_solver *s, long long i, int role, cudaStream_t st) {
     const SolverPtrs p = ptrs_of(s);
     const int g = s->AT.ntiles;
     if (g == 0) return;
@@ -1517,7 +1517,7 @@ void launch_P(sp_solver *s, int i, int role, cudaStream_t st) {
     }
 }
 
-void launch_D(sp_solver *s, int i, int role, cudaStream_t st) {
+void launch_D(sp_solver *s, long long i, int role, cudaStream_t st) {
     const SolverPtrs p = ptrs_of(s);
     const int g = s->A.ntiles;
     if (g == 0) return;
@@ -1571,7 +1571,7 @@ void launch_D(sp_solver *s, int i, int role, cudaStream_t st) {
     }
 }
 
-void launch_T(sp_solver *s, int i, cudaStream_t st) {
+void launch_T(sp_solver *s, long long i, cudaStream_t st) {
     const SolverPtrs p = ptrs_of(s);
     if (s->AT.ntiles == 0) return;
     CheckPassT o{};
@@ -1587,11 +1587,11 @@ void launch_T(sp_solver *s, int i, cudaStream_t st) {
 
 // One epoch of E iterations (the last is the check) on stream `st`. With timing
 // on, CUDA events bracket the P and D launches of sampled MID iterations.
-int enqueue_epoch(sp_solver *s, int E, cudaStream_t st, bool timed) {
+int enqueue_epoch(sp_solver *s, int64_t E, cudaStream_t st, bool timed) {
     int rc = SP_OK;
     const SolverPtrs p = ptrs_of(s);
     const int gn = grid_of(s->ctx, std::max(s->n, s->m));
-    for (int i = 0; i < E; ++i) {
+    for (int64_t i = 0; i < E; ++i) {
         const bool last = i == E - 1;
         const int role = last ? ROLE_CHECK : (i == 0 ? ROLE_FIRST : ROLE_MID);
         if (role == ROLE_MID && s->grid_ctas && !timed) {  // all MID iterations at once
@@ -1643,7 +1643,7 @@ int set_smem_limits() {
     return SP_OK;
 }
 
-int build_graph(sp_solver *s, int E, cudaGraphExec_t *out) {
+int build_graph(sp_solver *s, int64_t E, cudaGraphExec_t *out) {
     cudaStream_t st = s->ctx->stream;
     cudaGraph_t g;
     SP_CUDA_TRY(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
@@ -2125,7 +2125,7 @@ int power_iteration(sp_solver *s) {  // Solver::estimate_norm (solver.rs:215-242
         // pi_done tells a finished iteration from a stalled one: no error is left from before
         SP_CUDA_TRY(cudaMemsetAsync(s->d_st, 0, sizeof(DevState), st));
         const int rc = s->res_ctas ? res_launch(s, s->res_power, maxit)
-                                   : grid_launch(s, s->grid_power, (int)std::min<uint64_t>(maxit, INT32_MAX));
+                                   : grid_launch(s, s->grid_power, (long long)std::min<uint64_t>(maxit, INT32_MAX));
         if (rc) return rc;
     }
     DevState h{};  // with no iterations, λ stays 0 as in the reference
@@ -2371,7 +2371,7 @@ extern "C" int sp_solver_create(sp_ctx *ctx, const sp_lp *lp, const sp_solver_pa
 
 namespace sp {
 
-int epoch_graph(sp_solver *s, int E, cudaGraphExec_t *g) {
+int epoch_graph(sp_solver *s, int64_t E, cudaGraphExec_t *g) {
     auto it = s->graphs.find(E);
     if (it != s->graphs.end()) {
         *g = it->second;
@@ -2380,7 +2380,7 @@ int epoch_graph(sp_solver *s, int E, cudaGraphExec_t *g) {
     const double t0 = now_s();
     int rc = build_graph(s, E, g);
     if (rc) return rc;
-    if (getenv("SP_SETUP_TRACE")) fprintf(stderr, "solve graph(%d)    %8.2f ms\n", E, (now_s() - t0) * 1e3);
+    if (getenv("SP_SETUP_TRACE")) fprintf(stderr, "solve graph(%lld)    %8.2f ms\n", (long long)E, (now_s() - t0) * 1e3);
     s->graphs[E] = *g;
     return SP_OK;
 }
@@ -2408,7 +2408,7 @@ int res_launch_next(sp_solver *s, uint64_t n) {
 }
 
 // Enqueues one epoch (graph, or direct launches when timing samples are due).
-int launch_epoch(sp_solver *s, int E) {
+int launch_epoch(sp_solver *s, int64_t E) {
     cudaStream_t st = s->ctx->stream;
     if (res_epochs_on(s)) return res_launch_next(s, 1);
     if (s->timing_every > 0) {
@@ -2457,7 +2457,7 @@ extern "C" int sp_solver_run_epochs(sp_solver *s, uint64_t epochs) {
             e += n - 1;
             continue;
         }
-        if ((rc = launch_epoch(s, (int)E))) return rc;
+        if ((rc = launch_epoch(s, (int64_t)E))) return rc;
     }
     return SP_OK;
 }
@@ -2510,7 +2510,7 @@ extern "C" int sp_solver_solve(sp_solver *s, sp_solution_info *info) {
             if (several) {
                 if ((rc = res_launch_next(s, burst))) return rc;
                 burst = std::min(2 * burst, RES_MAX_EPOCHS);
-            } else if ((rc = launch_epoch(s, (int)E))) {
+            } else if ((rc = launch_epoch(s, (int64_t)E))) {
                 return rc;
             }
             const int slot = (int)(queued % ev.size());

@@ -60,7 +60,7 @@ struct IterScalars {
     double tau, sigma, w, rho;
 };
 
-__device__ __forceinline__ IterScalars iter_scalars(const SolverPtrs &s, int i) {
+__device__ __forceinline__ IterScalars iter_scalars(const SolverPtrs &s, long long i) {
     IterScalars r;
     const double omega = s.st->omega, eta = s.prm->eta;
     r.tau = eta / omega;  // solver.rs:333
@@ -90,7 +90,8 @@ struct PrimalPass {
     const Tile *tiles;
     const uint16_t *sched;  // null: rows in order
     SolverPtrs s;
-    int i, role;
+    long long i;
+    int role;
     IterScalars sc;
 
     __device__ bool setup() {
@@ -191,7 +192,8 @@ struct DualPass {
     const Tile *tiles;
     const uint16_t *sched;  // null: rows in order
     SolverPtrs s;
-    int i, role;
+    long long i;
+    int role;
     IterScalars sc;
 
     __device__ bool setup() {
@@ -303,7 +305,7 @@ struct CheckPassT {
     const Tile *tiles;
     const uint16_t *sched;  // null: rows in order
     SolverPtrs s;
-    int i;
+    long long i;
     double inv_tau;
 
     __device__ bool setup() {

@@ -17,7 +17,7 @@ struct ResLaunch {  // a kernel of the on-chip engine and its dynamic shared mem
     ResKernel f = nullptr;
     int smem = 0;
 };
-using GridKernel = void (*)(GridArgs, int);
+using GridKernel = void (*)(GridArgs, long long);
 struct GridLaunch {
     GridKernel f = nullptr;
     int smem = 0;
@@ -79,8 +79,8 @@ struct sp_solver {
     sp::DevState *h_st = nullptr;  // pinned, one slot per queued epoch
     sp_check_record *d_trace = nullptr;
     int64_t trace_cap = 0;
-    std::map<int, cudaGraphExec_t> graphs;  // epoch length -> instantiated graph
-    std::map<int, int64_t> graph_kernels;    // epoch length -> kernel nodes of its graph
+    std::map<int64_t, cudaGraphExec_t> graphs;  // epoch length -> instantiated graph
+    std::map<int64_t, int64_t> graph_kernels;  // epoch length -> kernel nodes of its graph
     uint64_t launched = 0;
     bool time_limited = false;
     double setup_s = 0, solve_s = 0;
