@@ -238,6 +238,12 @@ double sp_solver_bytes_per_iteration(sp_solver *s);
  * and all of them where sp_solver_set_timing has them launched one by one. */
 enum { SP_ENGINE_TILES = 0, SP_ENGINE_STREAM = 1, SP_ENGINE_SELL = 2 };
 int sp_solver_engines(sp_solver *s, int32_t out[4]);
+/* What runs an epoch's iterations: out[0] the engine, out[1] its CTAs (0 for launches), out[2]
+ * and out[3] what it keeps in shared memory in FP64 and in the FP32 phase (0 neither, 1 the row
+ * inputs, 2 the matrix entries too), out[4] the epochs so far that the grid engine left to
+ * launches because other streams' kernels held the SMs. */
+enum { SP_EPOCHS_LAUNCHED = 0, SP_EPOCHS_ON_CHIP = 1, SP_EPOCHS_GRID = 2 };
+int sp_solver_epoch_engine(sp_solver *s, int64_t out[5]);
 /* The floor a pass's random gathers set: the average time of a kernel that does only
  * those gathers (pass 0 primal: y through A'ᵀ's column indices; 1 dual: x̄ through A''s;
  * fp32 != 0: the mixed form's FP32 vectors), each through the pass's own index stream,

@@ -533,6 +533,17 @@ class Solver(_Handle):
         keys = ("primal_fp64", "primal_fp32", "dual_fp64", "dual_fp32")
         return {k: self.ENGINES[int(v)] for k, v in zip(keys, out)}
 
+    EPOCH_ENGINES = {0: "launched", 1: "on chip", 2: "grid"}
+
+    def epoch_engine(self) -> dict:
+        """What runs an epoch's iterations: 'engine' ('launched' | 'on chip' | 'grid'), its 'ctas',
+        what it keeps in shared memory in 'fp64' and in the 'fp32' phase (0 neither, 1 the row
+        inputs, 2 the matrix entries too), and the epochs that the grid engine has 'left' to
+        launches because other streams' kernels held the SMs."""
+        out = (C.c_int64 * 5)()
+        self._c(self.lib.sp_solver_epoch_engine(self.h, out))
+        return dict(zip(("engine", "ctas", "fp64", "fp32", "left"), (self.EPOCH_ENGINES[out[0]], *out[1:])))
+
     def gather_floor(self, kernel_id: int, fp32: bool = False, reps: int = 10) -> float:
         """Milliseconds of a kernel doing only pass `kernel_id`'s gathers (0 primal, 1 dual)
         through its own index stream: the floor its random gathers set."""

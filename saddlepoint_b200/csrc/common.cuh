@@ -141,7 +141,8 @@ struct DevState {
 // FP32 phase is taken to have stalled at its precision and the SpMV moves to FP64.
 constexpr int MIXED_STALL_CHECKS = 40;
 
-enum : int { ERR_NONE = 0, ERR_NUMERICAL_POWER = 1, ERR_NUMERICAL_ITERATES = 2, ERR_PIPELINE_STALL = 3, ERR_GRID_STALL = 4 };
+enum : int { ERR_NONE = 0, ERR_NUMERICAL_POWER = 1, ERR_NUMERICAL_ITERATES = 2, ERR_PIPELINE_STALL = 3, ERR_GRID_STALL = 4,
+             ERR_GRID_BUSY = 5 };  // ... BUSY: no failure, the host runs the epoch by launches (grid.cuh)
 
 // Elements of slack after the last row pointer / nonzero / vector entry of the
 // arrays the stream engine stages: a bulk copy rounds its range out to 16 bytes.

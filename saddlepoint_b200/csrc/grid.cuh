@@ -1,5 +1,4 @@
-// grid.cuh — a mid-sized LP on the whole chip: the FUSED iterations of an epoch in one
-// cooperative launch.
+// grid.cuh — a mid-sized LP on the whole chip: the FUSED iterations of an epoch in one launch.
 //
 // Between the LPs that one cluster holds (resident.cuh) and those whose passes fill the chip for
 // long, an iteration is two launches of 5-6 µs of which the work is a fraction, and each ends in
@@ -19,22 +18,32 @@
 
 namespace sp {
 
-// The grid's barrier: counts arrivals in global memory and waits for them. The launch is
-// cooperative, so every CTA is running. What was written to global memory before it is visible
-// after it. The wait is bounded (GRID_WAIT_NS; GRID_START_NS at a kernel's first barrier, which
-// waits until kernels of other streams, a batch's say, have left all SMs; or another CTA's giving up); a CTA that gives
-// up marks itself and all later barriers let it through, so that the kernel ends, and the
-// solve is reported as failed. 1.2 µs for 148 CTAs (B200); counting in two levels took 1.7.
-// A long wait is one for SMs that another kernel holds; it polls at intervals, since 144 CTAs
-// polling without pause slowed that kernel down eightfold (the set-up's norms: 6 ms to 46).
+// The grid's barrier: counts arrivals in global memory and waits for them. All CTAs are running
+// then (grid_start), and a CTA that runs goes on running. What was written to global memory
+// before it is visible after it. The wait is bounded (GRID_WAIT_NS, or another CTA's giving up);
+// a CTA that gives up marks itself and all later barriers let it through, so that the kernel
+// ends, and the solve is reported as failed. 1.2 µs for 148 CTAs (B200); counting in two levels
+// took 1.7.
+//
+// Whether all CTAs run is found out by the kernel's first wait, grid_start. The last CTA to start
+// decides for the launch; if another has waited GRID_START_NS for it, that one decides against
+// it, by compare-and-swap on one word, and all CTAs return without effect. That happens where
+// another stream's long kernel (a batch) holds SMs; the host then runs these iterations by
+// launches, which share the SMs (solver.cu: grid_resume). A cooperative launch would wait for
+// that kernel's end: 640 iterations of a 200k-nonzero LP beside a batch of 0.12 s solved over
+// and over took 0.9-1.3 s so, and take 0.01-0.24 s (the batch holds all SMs most of the time).
+// 0.1 to 1 ms of waiting did alike there, 3 ms and more worse; CTAs of a launch that has the SMs
+// start within some 10 µs.
 // The count wraps (148 arrivals twice an iteration: after 14.5M iterations of a launch), so
 // counts are compared by their difference, which is at most one barrier's arrivals; it starts
 // one below the wrap, so that every launch passes it.
-constexpr unsigned long long GRID_START_NS = 600000000000ull, GRID_WAIT_NS = 10000000000ull, GRID_SPIN_NS = 100000ull;
+constexpr unsigned long long GRID_START_NS = 300000ull, GRID_WAIT_NS = 10000000000ull, GRID_SPIN_NS = 100000ull;
 struct GridBar {
     unsigned count, alive;  // alive: 0 once a wait has given up
+    unsigned gate;          // GRID_GO or GRID_LEFT once the launch's fate is decided
 };
-constexpr unsigned GRID_COUNT0 = ~0u;  // both words at a launch's start (one fill)
+constexpr unsigned GRID_COUNT0 = ~0u;  // all words at a launch's start (one fill)
+constexpr unsigned GRID_LEFT = 0, GRID_GO = 1;
 __host__ __device__ constexpr bool grid_before(unsigned count, unsigned target) { return (int)(count - target) < 0; }
 static_assert(grid_before(GRID_COUNT0, GRID_COUNT0 + 148u) && grid_before(147u, 148u) && !grid_before(148u, 148u) &&
                   !grid_before(3u, GRID_COUNT0) && grid_before(0xfffffff0u, 16u),
@@ -43,6 +52,9 @@ struct GridState {
     GridBar *bar;
     unsigned passed;  // the count after the barriers so far
     int dead;         // a wait gave up
+    int left;         // the launch is left without effect
+    int leader;       // ... by this CTA
+    unsigned long long wait_ns;
 };
 
 __device__ __forceinline__ unsigned ld_acquire(const unsigned *p) {
@@ -51,7 +63,40 @@ __device__ __forceinline__ unsigned ld_acquire(const unsigned *p) {
     return v;
 }
 
-__device__ __forceinline__ void grid_sync(GridState &g, unsigned long long limit = GRID_WAIT_NS) {  // g: a shared variable
+// Whether all CTAs have started, the same answer in all of them: the last one to come decides for
+// it, or the first whose wait for it exceeds `limit` against it.
+__device__ __forceinline__ bool grid_start(GridState &g, unsigned long long limit) {  // g: a shared variable
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        g.passed += gridDim.x;
+        unsigned before, gate = GRID_COUNT0;
+        asm volatile("atom.acq_rel.gpu.global.add.u32 %0, [%1], 1;" : "=r"(before) : "l"(&g.bar->count) : "memory");
+        if (before + 1 == g.passed) {
+            __threadfence();  // all CTAs' writes before the decision
+            gate = atomicCAS(&g.bar->gate, GRID_COUNT0, GRID_GO);
+            if (gate == GRID_COUNT0) gate = GRID_GO;
+        }
+        const unsigned long long t0 = global_ns();
+        while (gate == GRID_COUNT0 && (gate = ld_acquire(&g.bar->gate)) == GRID_COUNT0) {
+            const unsigned long long waited = global_ns() - t0;
+            if (waited >= limit) {
+                gate = atomicCAS(&g.bar->gate, GRID_COUNT0, GRID_LEFT);
+                if (gate == GRID_COUNT0) {
+                    gate = GRID_LEFT;
+                    g.leader = 1;
+                }
+            } else if (waited > GRID_SPIN_NS) {
+                __nanosleep(1000);
+            }
+        }
+        __threadfence();  // ... and after it
+        g.left = gate == GRID_LEFT;
+    }
+    __syncthreads();
+    return !g.left;
+}
+
+__device__ __forceinline__ void grid_sync(GridState &g) {  // g: a shared variable
     __syncthreads();
     if (threadIdx.x == 0 && !g.dead) {
         const unsigned target = g.passed + gridDim.x;
@@ -60,7 +105,7 @@ __device__ __forceinline__ void grid_sync(GridState &g, unsigned long long limit
             const unsigned long long t0 = global_ns();
             while (grid_before(ld_acquire(&g.bar->count), target)) {
                 const unsigned long long waited = global_ns() - t0;
-                if (!ld_acquire(&g.bar->alive) || waited > limit) {
+                if (!ld_acquire(&g.bar->alive) || waited >= g.wait_ns) {
                     atomicExch(&g.bar->alive, 0u);
                     g.dead = 1;
                     break;
@@ -112,6 +157,7 @@ struct GridArgs {
     float *y32, *xbar32;
     double *contrib, *ppart;        // the power iteration's
     GridBar *bar;                   // all ones before each launch
+    unsigned long long start_ns, wait_ns;  // limits of the first wait and of the others
     int mixed;
 };
 
@@ -123,6 +169,7 @@ __host__ __device__ inline GridPlaces<VS, ES, PT, PA> grid_places(const GridArgs
 struct GridShared {
     ResSide<int> A, T;
     GridState grid;
+    int due;
     double wtab[RES_WTAB];
     double sh[RES_GROUPS * (NT / 32) + 1];
 };
@@ -132,7 +179,7 @@ template <bool VS, bool ES, int PT, int PA>
 __device__ inline void grid_open(GridShared &sh, const GridPlaces<VS, ES, PT, PA> &L, const GridArgs &a) {
     const int c = (int)blockIdx.x;
     if (threadIdx.x == 0) {
-        sh.grid = GridState{a.bar, GRID_COUNT0, 0};
+        sh.grid = GridState{a.bar, GRID_COUNT0, 0, 0, 0, a.wait_ns};
         sh.A = res_side(a.A, c, L.tasksA, L.wtA);
         sh.T = res_side(a.T, c, L.tasksT, L.wtT);
     }
@@ -309,10 +356,14 @@ __global__ void __launch_bounds__(RES_BT, 1) k_grid_mid(const __grid_constant__ 
     using VT = typename std::conditional<LO, float, double>::type;
     using P = GridPlaces<VS, ES, PT, PA>;
     __shared__ GridShared sh;
-    {
+    // The same for every thread of a CTA. A CTA that starts after the launch was left may see
+    // the state that says so.
+    if (threadIdx.x == 0) {
         const DevState *st = a.g.st;
-        if (st->done || LO != (a.mixed && !st->fp64)) return;  // the same for every CTA
+        sh.due = !st->done && LO == (a.mixed && !st->fp64);
     }
+    __syncthreads();
+    if (!sh.due) return;
     const P L = grid_places<VS, ES, PT, PA>(a, LO);
     grid_open(sh, L, a);
     const VT *vT, *vA;
@@ -411,7 +462,13 @@ __global__ void __launch_bounds__(RES_BT, 1) k_grid_mid(const __grid_constant__ 
         a.y[k] = yn;
         if constexpr (LO) gy[k] = (float)yn;
     };
-    grid_sync(sh.grid, GRID_START_NS);
+    if (!grid_start(sh.grid, a.start_ns)) {  // so far nothing but this engine's own vectors was written
+        if (threadIdx.x == 0 && sh.grid.leader) {
+            a.g.st->error = ERR_GRID_BUSY;
+            a.g.st->done = 1;
+        }
+        return;
+    }
     const unsigned long long k0 = a.g.st->k;
 #pragma unroll 1
     for (unsigned long long i = 1; i + 1 < (unsigned long long)E && !sh.grid.dead; ++i) {
@@ -504,7 +561,13 @@ __global__ void __launch_bounds__(RES_BT, 1) k_grid_power(const __grid_constant_
     double scale = 1.0 / sqrt(s[0]), lambda = 0.0;
     int iters = 0, error = ERR_NONE;
     bool done = false;
-    grid_sync(sh.grid, GRID_START_NS);
+    if (!grid_start(sh.grid, a.start_ns)) {
+        if (threadIdx.x == 0 && sh.grid.leader) {
+            a.g.st->error = ERR_GRID_BUSY;
+            a.g.st->pi_done = 1;
+        }
+        return;
+    }
     while (!done && !sh.grid.dead) {
         grid_rows(EA, L.tasksA, a0, a1, [&](double x, double g) { return x * (g * scale); },
                   [&](int ty, int tz, double q) {

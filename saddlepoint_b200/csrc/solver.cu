@@ -1108,6 +1108,7 @@ int res_build(sp_solver *s, const sp_lp *lp, const std::vector<int> &rp_t) {
         const int in = res_solver_places(a.A, a.T, lo, true).total, out = res_solver_places(a.A, a.T, lo, false).total;
         if (out > RES_SMEM_MAX) return SP_OK;
         const bool fits = in <= RES_SMEM_MAX;
+        s->epoch_level[lo] = fits ? 2 : 1;
         s->res_epochs[lo] = ResLaunch{one ? res_kernel_of<1>(lo, fits) : res_kernel_of<RES_CLUSTER>(lo, fits), fits ? in : out};
         if (lo == 0)
             s->res_power = ResLaunch{one ? (fits ? k_res_power<1, true> : k_res_power<1, false>)
@@ -1206,12 +1207,14 @@ void split_ranges(int64_t len, const F &body) {
 constexpr int GRID_PT = 1024, GRID_PA = 512;     // columns and rows of a CTA with entries in shared memory
 constexpr int GRID_PT2 = 2560, GRID_PA2 = 1280;  // ... without
 
+constexpr uint64_t GRID_BACKOFF = 64;            // epochs by launches after one that found no SMs (grid_resume)
+
+// Not a cooperative launch: grid_start finds out in the kernel whether all CTAs run.
 int grid_launch(const sp_solver *s, const GridLaunch &l, long long n) {
     cudaStream_t st = s->ctx->stream;
     SP_CUDA_TRY(cudaMemsetAsync(s->grid.bar, GRID_COUNT0 & 0xff, sizeof(GridBar), st));
     void *args[] = {(void *)&s->grid, (void *)&n};
-    SP_CUDA_TRY(cudaLaunchCooperativeKernel((const void *)l.f, dim3((unsigned)s->grid_ctas), dim3(RES_BT), args,
-                                            (size_t)l.smem, st));
+    SP_CUDA_TRY(cudaLaunchKernel((const void *)l.f, dim3((unsigned)s->grid_ctas), dim3(RES_BT), args, (size_t)l.smem, st));
     return SP_OK;
 }
 
@@ -1276,8 +1279,8 @@ int grid_order(sp_solver *s, const DevCsr &D, const ResSrc<int> &M, const int *f
 // 96 | 115 (mixed 3.4M 44.5 | 51.3): hence GRID_MAX_LONG for rows of GRID_LONG_ROW on average.
 //
 // The power iteration (ms, launches | grid): 80k 0.88 | 0.48, 200k 3.67 | 2.20, 500k 3.62 | 2.18,
-// 1M 5.35 | 3.80, 2M 5.06 | 4.48, 3M 10.3 | 10.6. From 1M on the norms' chains of additions,
-// which hold SMs beside it that the grid has to wait for, count: hence GRID_POWER_MAX_NNZ.
+// 1M 5.35 | 3.80, 2M 5.06 | 4.48, 3M 10.3 | 10.6 (a grid that waits for its SMs). From 1M on the
+// norms' chains of additions hold SMs beside it for milliseconds: hence GRID_POWER_MAX_NNZ.
 constexpr int64_t GRID_MAX_NNZ = 3 << 23, GRID_MAX_LONG = 1 << 21, GRID_LONG_ROW = 128, GRID_POWER_MAX_NNZ = 1 << 19;
 struct GridPlan {
     std::thread th;
@@ -1297,9 +1300,6 @@ struct GridPlan {
         if (nnz < 1 || m < 1 || n < 1 || s->A.nlong) return SP_OK;
         if (!forced && (s->ctx->shared || nnz > GRID_MAX_NNZ || (nnz > GRID_MAX_LONG && nnz / m >= GRID_LONG_ROW)))
             return SP_OK;
-        int coop = 0;
-        SP_CUDA_TRY(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, s->ctx->device));
-        if (!coop) return SP_OK;
         ctas = (int)std::min<int64_t>(s->ctx->sms, std::max<int64_t>(4, nnz / 1000));
         const int64_t *rp_a = lp->a.row_ptr;
         const int *rpt = rp_t.data();
@@ -1367,6 +1367,7 @@ int grid_build(sp_solver *s, GridPlan &plan_of) {
             l = {lo ? k_grid_mid<true, false, false, 0, 0> : k_grid_mid<false, false, false, 0, 0>, none};
         else
             return SP_OK;
+        s->epoch_level[lo] = l.smem == none ? 0 : l.smem == rows ? 1 : 2;
         if (lo == 0 && s->nnz <= GRID_POWER_MAX_NNZ) {  // the power iteration has no row inputs
             const int pe = grid_places<false, true, 0, 0>(a, false).total, pn = grid_places<false, false, 0, 0>(a, false).total;
             s->grid_power = pe <= RES_SMEM_MAX ? GridLaunch{k_grid_power<true>, pe} : GridLaunch{k_grid_power<false>, pn};
@@ -1453,6 +1454,13 @@ int grid_build(sp_solver *s, GridPlan &plan_of) {
     a.xbar32 = s->mixed ? a.y32 + M + GRID_ONES : nullptr;
     a.contrib = (double *)(d + contrib);
     a.bar = (GridBar *)(d + bar);
+    a.start_ns = GRID_START_NS;
+    a.wait_ns = GRID_WAIT_NS;
+    // test knob of the waits' ends: the first wait, or one between passes, gives up at once
+    if (const char *w = getenv("SP_TEST_GRID_WAIT")) {
+        if (!strcmp(w, "start")) a.start_ns = 0;
+        if (!strcmp(w, "pass")) a.wait_ns = 0;
+    }
     a.ppart = s->ppart;
     a.mixed = s->mixed;
     a.g = ptrs_of(s);
@@ -1585,16 +1593,17 @@ void launch_T(sp_solver *s, long long i, cudaStream_t st) {
     launch_tiles(s->ctx->sms, s->ctx->d_tiles, s->AT.ntiles, smem_T(), st, o);
 }
 
-// One epoch of E iterations (the last is the check) on stream `st`. With timing
-// on, CUDA events bracket the P and D launches of sampled MID iterations.
-int enqueue_epoch(sp_solver *s, int64_t E, cudaStream_t st, bool timed) {
+// One epoch of E iterations (the last is the check) on stream `st`, from iteration `from` on;
+// grid: the MID iterations on the grid engine. With timing on, CUDA events bracket the P and D
+// launches of sampled MID iterations.
+int enqueue_epoch(sp_solver *s, int64_t E, cudaStream_t st, bool timed, bool grid, int64_t from = 0) {
     int rc = SP_OK;
     const SolverPtrs p = ptrs_of(s);
     const int gn = grid_of(s->ctx, std::max(s->n, s->m));
-    for (int64_t i = 0; i < E; ++i) {
+    for (int64_t i = from; i < E; ++i) {
         const bool last = i == E - 1;
         const int role = last ? ROLE_CHECK : (i == 0 ? ROLE_FIRST : ROLE_MID);
-        if (role == ROLE_MID && s->grid_ctas && !timed) {  // all MID iterations at once
+        if (role == ROLE_MID && grid) {  // all MID iterations at once
             if (!rc && s->mixed) rc = grid_launch(s, s->grid_mid[1], E);
             if (!rc) rc = grid_launch(s, s->grid_mid[0], E);
             i = E - 2;
@@ -1647,7 +1656,7 @@ int build_graph(sp_solver *s, int64_t E, cudaGraphExec_t *out) {
     cudaStream_t st = s->ctx->stream;
     cudaGraph_t g;
     SP_CUDA_TRY(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
-    const int rc = enqueue_epoch(s, E, st, false);
+    const int rc = enqueue_epoch(s, E, st, false, s->grid_ctas > 0);
     SP_CUDA_TRY(cudaStreamEndCapture(st, &g));
     if (rc) {
         cudaGraphDestroy(g);
@@ -2111,12 +2120,13 @@ int power_iteration(sp_solver *s) {  // Solver::estimate_norm (solver.rs:215-242
         s->norm_est = 1.0;
         return SP_OK;
     }
-    const bool once = s->res_ctas || (s->grid_ctas && s->grid_power.f);  // all iterations in one launch
-    if (!once) {
+    bool once = s->res_ctas || (s->grid_ctas && s->grid_power.f);  // all iterations in one launch
+    auto start = [&] {
         k_power_fill<<<grid_of(s->ctx, s->n), NT, 0, st>>>(s->pv, s->n);
         k_power_init<<<1, NT, 0, st>>>(s->n, s->ppart);
         k_power_start<<<1, 32, 0, st>>>(s->ppart, s->d_st);
-    }
+    };
+    if (!once) start();
     const uint64_t maxit = s->prm.power_iterations;
     PowerA a{s->A.rp, s->A.ci, s->A.v, s->A.tiles, s->pv, s->ptmp, s->d_st, 0.0};
     PowerT t{s->AT.rp, s->AT.ci, s->AT.v, s->AT.tiles, s->ptmp, s->pv, s->ppart, s->d_st};
@@ -2142,6 +2152,14 @@ int power_iteration(sp_solver *s) {  // Solver::estimate_norm (solver.rs:215-242
         done_it += c;
         SP_CUDA_TRY(cudaMemcpyAsync(&h, s->d_st, sizeof(DevState), cudaMemcpyDeviceToHost, st));
         SP_CUDA_TRY(cudaStreamSynchronize(st));
+        if (h.error == ERR_GRID_BUSY) {  // the grid found no SMs: by launches, from the start
+            SP_CUDA_TRY(cudaMemsetAsync(s->d_st, 0, sizeof(DevState), st));
+            h = DevState{};
+            once = false;
+            start();
+            done_it = 0;
+            continue;
+        }
         if (h.pi_done) break;
     }
     if (h.error == ERR_GRID_STALL) return fail(SP_ERR_CUDA, GRID_STALL_MESSAGE);
@@ -2212,6 +2230,8 @@ extern "C" int sp_solver_reset(sp_solver *s) {
     SP_CUDA_TRY(cudaStreamSynchronize(st));
     s->launched = 0;
     s->time_limited = false;
+    s->grid_pause = 0;
+    s->grid_backoff = GRID_BACKOFF;
     return SP_OK;
 }
 
@@ -2407,12 +2427,13 @@ int res_launch_next(sp_solver *s, uint64_t n) {
     return rc;
 }
 
-// Enqueues one epoch (graph, or direct launches when timing samples are due).
+// Enqueues one epoch: its graph, or direct launches when timing samples are due and while the
+// grid engine pauses (a second graph would not do: to make one waits for all streams' kernels).
 int launch_epoch(sp_solver *s, int64_t E) {
     cudaStream_t st = s->ctx->stream;
     if (res_epochs_on(s)) return res_launch_next(s, 1);
-    if (s->timing_every > 0) {
-        const int rc = enqueue_epoch(s, E, st, true);
+    if (s->timing_every > 0 || s->grid_pause > 0) {
+        const int rc = enqueue_epoch(s, E, st, s->timing_every > 0, false);
         if (rc) return rc;
     } else {
         cudaGraphExec_t g;
@@ -2422,7 +2443,44 @@ int launch_epoch(sp_solver *s, int64_t E) {
     }
     SP_CUDA_TRY(cudaGetLastError());
     s->launched += (uint64_t)E;
+    if (s->grid_pause > 0) --s->grid_pause;
     return SP_OK;
+}
+
+// The state h of an idle stream says that the grid engine left an epoch after its first
+// iteration (ERR_GRID_BUSY; the epochs behind it returned at once): the rest of that epoch by
+// launches, as the next ones. Each time that this happens the engine is tried again after
+// twice as many epochs, so that what the vain waits take stays small.
+int grid_resume(sp_solver *s, DevState h) {
+    cudaStream_t st = s->ctx->stream;
+    h.done = 0;
+    h.error = ERR_NONE;
+    SP_CUDA_TRY(cudaMemcpyAsync(s->d_st, &h, sizeof h, cudaMemcpyHostToDevice, st));
+    s->launched = h.total;
+    const uint64_t E = next_epoch(s);
+    const int rc = enqueue_epoch(s, (int64_t)E, st, false, false, 1);
+    if (rc) return rc;
+    SP_CUDA_TRY(cudaGetLastError());
+    s->launched += E;
+    s->grid_left += 1;
+    s->grid_pause = s->grid_backoff;
+    s->grid_backoff = std::min<uint64_t>(2 * s->grid_backoff, 1 << 20);
+    return SP_OK;
+}
+
+// The state after everything that was queued, epochs that the grid engine left included.
+int settle(sp_solver *s, DevState *h) {
+    int rc;
+    for (;;) {
+        SP_CUDA_TRY(cudaMemcpyAsync(s->h_st, s->d_st, sizeof(DevState), cudaMemcpyDeviceToHost, s->ctx->stream));
+        SP_CUDA_TRY(cudaStreamSynchronize(s->ctx->stream));
+        *h = *s->h_st;
+        if (h->error != ERR_GRID_BUSY) return SP_OK;
+        const uint64_t queued = s->launched;
+        if ((rc = grid_resume(s, *h))) return rc;
+        while (s->launched < queued)
+            if ((rc = launch_epoch(s, (int64_t)next_epoch(s)))) return rc;
+    }
 }
 
 void fill_info(sp_solver *s, const DevState &h, sp_solution_info *info) {
@@ -2466,8 +2524,8 @@ extern "C" int sp_solver_sync(sp_solver *s) {
     if (!s) return SP_ERR_INVALID;
     int rc = enter(s->ctx);
     if (rc) return rc;
-    SP_CUDA_TRY(cudaStreamSynchronize(s->ctx->stream));
-    return SP_OK;
+    DevState h;
+    return settle(s, &h);
 }
 
 extern "C" int sp_solver_solve(sp_solver *s, sp_solution_info *info) {
@@ -2523,6 +2581,16 @@ extern "C" int sp_solver_solve(sp_solver *s, sp_solution_info *info) {
         SP_CUDA_TRY(cudaEventSynchronize(ev[slot]));
         last = s->h_st[slot];
         ++seen;
+        if (last.error == ERR_GRID_BUSY) {  // as are the states behind it
+            SP_CUDA_TRY(cudaStreamSynchronize(st));
+            seen = queued;
+            if ((rc = grid_resume(s, last))) return rc;
+            const int next = (int)(queued % ev.size());
+            SP_CUDA_TRY(cudaMemcpyAsync(&s->h_st[next], s->d_st, sizeof(DevState), cudaMemcpyDeviceToHost, st));
+            SP_CUDA_TRY(cudaEventRecord(ev[next], st));
+            ++queued;
+            continue;
+        }
         if (s->prm.log_every_checks > 0 && last.checks > logged_checks && last.checks % s->prm.log_every_checks == 0) {
             logged_checks = last.checks;
             fprintf(stderr, "%9llu %14.6e %14.6e %9.2e %9.2e %9.2e %9.2e %5llu %8.2fs %7llu %9.2e\n",
@@ -2536,9 +2604,7 @@ extern "C" int sp_solver_solve(sp_solver *s, sp_solution_info *info) {
             stop = true;
         }
     }
-    SP_CUDA_TRY(cudaStreamSynchronize(st));
-    SP_CUDA_TRY(cudaMemcpy(s->h_st, s->d_st, sizeof(DevState), cudaMemcpyDeviceToHost));
-    last = s->h_st[0];
+    if ((rc = settle(s, &last))) return rc;
     s->solve_s = now_s() - t0;
     if (last.error == ERR_NUMERICAL_ITERATES) return fail(SP_ERR_NUMERICAL, "numerical breakdown: iterates are not finite");
     if (last.error == ERR_GRID_STALL) return fail(SP_ERR_CUDA, GRID_STALL_MESSAGE);
@@ -2553,9 +2619,8 @@ extern "C" int sp_solver_info(sp_solver *s, sp_solution_info *info) {
     if (!s || !info) return SP_ERR_INVALID;
     int rc = enter(s->ctx);
     if (rc) return rc;
-    SP_CUDA_TRY(cudaStreamSynchronize(s->ctx->stream));
     DevState h;
-    SP_CUDA_TRY(cudaMemcpy(&h, s->d_st, sizeof h, cudaMemcpyDeviceToHost));
+    if ((rc = settle(s, &h))) return rc;
     fill_info(s, h, info);
     return SP_OK;
 }
@@ -2565,6 +2630,8 @@ extern "C" int sp_solver_download(sp_solver *s, double *x, double *y) {
     int rc = enter(s->ctx);
     if (rc) return rc;
     cudaStream_t st = s->ctx->stream;
+    DevState h;
+    if (s->grid_ctas && (rc = settle(s, &h))) return rc;
     if (!s->out_x) {
         if ((rc = dalloc(&s->out_x, s->n)) || (rc = dalloc(&s->out_y, s->m))) return rc;
     }
@@ -2580,9 +2647,8 @@ extern "C" int sp_solver_trace(sp_solver *s, sp_check_record *out, int64_t cap, 
     if (!s || !len) return SP_ERR_INVALID;
     int rc = enter(s->ctx);
     if (rc) return rc;
-    SP_CUDA_TRY(cudaStreamSynchronize(s->ctx->stream));
     DevState h;
-    SP_CUDA_TRY(cudaMemcpy(&h, s->d_st, sizeof h, cudaMemcpyDeviceToHost));
+    if ((rc = settle(s, &h))) return rc;
     const int64_t avail = std::min<int64_t>((int64_t)h.trace_len, s->trace_cap);
     *len = avail;
     const int64_t k = std::min(avail, cap);
@@ -2692,6 +2758,16 @@ extern "C" int sp_solver_engines(sp_solver *s, int32_t out[4]) {
     if (!s || !out) return SP_ERR_INVALID;
     const int v[4] = {s->sv_p64, s->sv_p32, s->sv_d64, s->sv_d32};
     for (int k = 0; k < 4; ++k) out[k] = v[k] < 0 ? SP_ENGINE_TILES : (v[k] == ENGINE_SELL ? SP_ENGINE_SELL : SP_ENGINE_STREAM);
+    return SP_OK;
+}
+
+extern "C" int sp_solver_epoch_engine(sp_solver *s, int64_t out[5]) {
+    if (!s || !out) return SP_ERR_INVALID;
+    out[0] = s->res_ctas ? SP_EPOCHS_ON_CHIP : s->grid_ctas ? SP_EPOCHS_GRID : SP_EPOCHS_LAUNCHED;
+    out[1] = s->res_ctas ? s->res_ctas : s->grid_ctas;
+    out[2] = out[1] ? s->epoch_level[0] : 0;
+    out[3] = out[1] && s->mixed ? s->epoch_level[1] : 0;
+    out[4] = s->grid_left;
     return SP_OK;
 }
 

@@ -50,6 +50,11 @@ struct sp_solver {
     void *grid_slots[6] = {};
     sp::GridArgs grid{};
     sp::GridLaunch grid_mid[2], grid_power;  // an epoch's iterations in FP64 and in the FP32 phase
+    // the next grid_pause epochs run by launches, since the grid engine found no SMs for one;
+    // after the next such epoch grid_backoff do
+    uint64_t grid_pause = 0, grid_backoff = 0;
+    int epoch_level[2] = {};  // what the epoch engine keeps in shared memory (sp_solver_epoch_engine)
+    int64_t grid_left = 0;  // epochs that were left so, for sp_solver_epoch_engine
     double *contrib = nullptr;   // [NP_D][m] row contributions of the check's dual pass on the SELL copy
     int64_t m = 0, n = 0, nnz = 0;
     double c0 = 0.0;
