@@ -2468,13 +2468,18 @@ int grid_resume(sp_solver *s, DevState h) {
     return SP_OK;
 }
 
-// The state after everything that was queued, epochs that the grid engine left included.
+constexpr const char *PIPELINE_STALL_MESSAGE = "a bulk copy of the pass pipeline did not complete within its wait limit";
+
+// The state after everything that was queued, epochs that the grid engine left included. A wait
+// that gave up is an error here, whichever call asks: the iterates are not to be used.
 int settle(sp_solver *s, DevState *h) {
     int rc;
     for (;;) {
         SP_CUDA_TRY(cudaMemcpyAsync(s->h_st, s->d_st, sizeof(DevState), cudaMemcpyDeviceToHost, s->ctx->stream));
         SP_CUDA_TRY(cudaStreamSynchronize(s->ctx->stream));
         *h = *s->h_st;
+        if (h->error == ERR_GRID_STALL) return fail(SP_ERR_CUDA, GRID_STALL_MESSAGE);
+        if (h->error == ERR_PIPELINE_STALL) return fail(SP_ERR_CUDA, PIPELINE_STALL_MESSAGE);
         if (h->error != ERR_GRID_BUSY) return SP_OK;
         const uint64_t queued = s->launched;
         if ((rc = grid_resume(s, *h))) return rc;
@@ -2607,9 +2612,6 @@ extern "C" int sp_solver_solve(sp_solver *s, sp_solution_info *info) {
     if ((rc = settle(s, &last))) return rc;
     s->solve_s = now_s() - t0;
     if (last.error == ERR_NUMERICAL_ITERATES) return fail(SP_ERR_NUMERICAL, "numerical breakdown: iterates are not finite");
-    if (last.error == ERR_GRID_STALL) return fail(SP_ERR_CUDA, GRID_STALL_MESSAGE);
-    if (last.error == ERR_PIPELINE_STALL)
-        return fail(SP_ERR_CUDA, "a bulk copy of the pass pipeline did not complete within its wait limit");
     if (!last.done && !s->time_limited) s->time_limited = true;  // only reachable with an exhausted limit
     fill_info(s, last, info);
     return SP_OK;
@@ -2631,7 +2633,7 @@ extern "C" int sp_solver_download(sp_solver *s, double *x, double *y) {
     if (rc) return rc;
     cudaStream_t st = s->ctx->stream;
     DevState h;
-    if (s->grid_ctas && (rc = settle(s, &h))) return rc;
+    if ((rc = settle(s, &h))) return rc;
     if (!s->out_x) {
         if ((rc = dalloc(&s->out_x, s->n)) || (rc = dalloc(&s->out_y, s->m))) return rc;
     }

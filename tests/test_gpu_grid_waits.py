@@ -75,6 +75,62 @@ def test_every_read_finds_the_epochs_that_were_left(read, left_at_start, monkeyp
         np.testing.assert_equal(a, b)
 
 
+READS = {
+    "solve": lambda s: s.solve(),
+    "sync": lambda s: s.sync(),
+    "info": lambda s: s.info(),
+    "download": lambda s: s.download(),
+    "trace": lambda s: s.trace(),
+}
+
+
+def assert_every_read_fails(s, message):
+    for name, read in READS.items():
+        with pytest.raises(sp().SolveError) as e:
+            read(s)
+        assert e.value.code == 1 and message in str(e.value), name
+
+
+@pytest.mark.parametrize("mixed", [False, True])
+def test_a_stalled_barrier_is_an_error_of_every_read(mixed, monkeypatch, gpu_backend):
+    """The waits between passes give up at once: no caller gets the unfinished iterates as a
+    result. A new solver of the same context gives a clean solve's bits."""
+    lp = sp().generate_random_lp(24, 60000, 120000, (5, 5))  # its power iteration runs by launches
+    p = params(640, precision=sp().Precision.Mixed if mixed else sp().Precision.FP64)
+    clean = solve_with("tiles", lp, p, gpu_backend)
+    monkeypatch.setenv("SP_TEST_GRID_WAIT", "pass")
+    s = sp().Solver(lp, p, gpu_backend)
+    monkeypatch.delenv("SP_TEST_GRID_WAIT")
+    assert s.epoch_engine()["engine"] == "grid"
+    for _ in range(2):
+        s.run_epochs(3)
+        assert_every_read_fails(s, "the grid's barrier did not complete within its wait limit")
+        s.reset()
+    s.close()
+    assert_identical(sp().solve(lp, p, gpu_backend), clean)
+
+
+def test_a_stalled_barrier_of_the_power_iteration_is_an_error(monkeypatch, gpu_backend):
+    lp = sp().generate_random_lp(24, 6000, 12000, (5, 5))
+    monkeypatch.setenv("SP_TEST_GRID_WAIT", "pass")
+    with pytest.raises(sp().SolveError) as e:
+        sp().Solver(lp, params(640), gpu_backend)
+    assert e.value.code == 1 and "the grid's barrier" in str(e.value)
+
+
+def test_a_stalled_bulk_copy_is_an_error_of_every_read(monkeypatch, gpu_backend):
+    """The stream engine's stall (its own test knob) on the same paths."""
+    lp = sp().generate_powerlaw_lp(6, 4000, 8000, 60000, 1.5, 2, 1500)
+    monkeypatch.setenv("SP_PASS_ENGINE", "stream")
+    monkeypatch.setenv("SP_TEST_STREAM_WITHHOLD", "0")
+    s = sp().Solver(lp, params(640), gpu_backend)
+    monkeypatch.delenv("SP_PASS_ENGINE")
+    monkeypatch.delenv("SP_TEST_STREAM_WITHHOLD")
+    s.run_epochs(2)
+    assert_every_read_fails(s, "a bulk copy of the pass pipeline did not complete")
+    s.close()
+
+
 def test_a_solve_beside_a_long_batch_runs(gpu_backend):
     """A kernel of another stream that holds an SM for seconds: the solve neither waits for it nor
     fails, and ends at its time limit; then the engine has the SMs again."""
