@@ -255,9 +255,10 @@ __device__ void batch_tiles_solve(const BatchArgs &A, const BatchInst &I, const 
             st.error = ERR_NUMERICAL_POWER;
         }
     }
-    for (int j = tid; j < n; j += BT) S.x[j] = S.xa[j] = 0.0;
+    // x_t and y_t too: a solve that ends before its first pass returns them
+    for (int j = tid; j < n; j += BT) S.x[j] = S.xa[j] = S.xt[j] = 0.0;
     for (int i = tid; i < m; i += BT) {
-        S.y[i] = S.ya[i] = 0.0;
+        S.y[i] = S.ya[i] = S.yt[i] = 0.0;
         if (mixed) S.y32[i] = 0.0f;
     }
     __syncthreads();
@@ -605,9 +606,9 @@ __device__ void batch_solve_one(const BatchArgs &A, int id, double *sh, DevState
             st.error = ERR_NUMERICAL_POWER;
         }
     }
-    for (int j = tid; j < n; j += BT) x[j] = xa[j] = 0.0;
+    for (int j = tid; j < n; j += BT) x[j] = xa[j] = xt[j] = 0.0;
     for (int i = tid; i < m; i += BT) {
-        y[i] = ya[i] = 0.0;
+        y[i] = ya[i] = yt[i] = 0.0;
         if (mixed) y32[i] = 0.0f;
     }
     __syncthreads();

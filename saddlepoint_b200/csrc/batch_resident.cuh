@@ -408,7 +408,7 @@ __device__ __noinline__ void res_batch_setup(const BatchArgs &A, const BatchRes 
         const_cast<double *>(S.lv)[k] = lo;
         const_cast<double *>(S.uv)[k] = hi;
         vec.df[k] = 1.0 / (f * os);
-        S.x[k] = S.xa[k] = 0.0;
+        S.x[k] = S.xa[k] = S.xt[k] = 0.0;  // x_t and y_t: a solve that ends before its first pass returns them
     }
     for (int k = MA.p0 + threadIdx.x; k < MA.p1; k += RES_BT) {
         const int i = MA.perm[k];
@@ -421,7 +421,7 @@ __device__ __noinline__ void res_batch_setup(const BatchArgs &A, const BatchRes 
         const_cast<double *>(S.lc)[k] = lo;
         const_cast<double *>(S.uc)[k] = hi;
         vec.pf[k] = 1.0 / (f * bs);
-        S.ya[k] = 0.0;
+        S.ya[k] = S.yt[k] = 0.0;
     }
     res_sync<NC>();
     if (D.nnz > 0) res_power<NC, ES>(s, L, A.power_iterations, ppart);

@@ -45,3 +45,26 @@ def test_each_class_gives_the_solo_solve(mixed, gpu_backend):
             x, y = b.solution(i)
             assert res[i].iterations == solo.iterations == 200 and res[i].objective == solo.objective, i
             assert np.array_equal(x, solo.x) and np.array_equal(y, solo.y), i
+
+
+@pytest.mark.parametrize("m,ctas", [(40, 1), (700, 1), (1400, 2), (2300, None)])
+def test_an_instance_without_a_first_iteration_has_a_zero_solution(m, ctas, gpu_backend, monkeypatch):
+    """Coefficients of zero: the power iteration collapses before any iterate exists. The solution
+    is zero, not what the scratch held of another instance, in any mix and on every solve."""
+    monkeypatch.setenv("SP_BATCH_HANDOFF_S", "0")
+    bad = sp().generate_random_lp(5, m, 2 * m, (2, 2))
+    bad.values = np.zeros_like(bad.values)
+    # others of its class that run before it on the same clusters, and smaller ones
+    others = [sp().generate_random_lp(200 + i, m, 2 * m, (4, 6)) for i in range(160)]
+    others += [sp().generate_random_lp(500 + i, 30, 60, (3, 5)) for i in range(5)]
+    p = sp().SolverParams(tolerance=0.0, infeasibility_tolerance=0.0, max_iterations=64)
+    for lps, at in (([bad], 0), (others + [bad], len(others))):
+        b = sp().BatchSolver(lps, p, gpu_backend)
+        assert (b.engine(at) or (None,))[0] == ctas
+        for _ in range(2):
+            res, _ = b.solve()
+            assert res[at].status == -2  # a numerical breakdown of the power iteration
+            x, y = b.solution(at)
+            assert not x.any() and not y.any()
+            assert all(r.status == 3 for i, r in enumerate(res) if i != at)
+        b.close()
