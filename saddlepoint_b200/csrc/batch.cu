@@ -143,10 +143,6 @@ int calibrate(sp_ctx *ctx, TuneTable *T) {
             const BatchInst &I = inst[c];
             A2.base.max_iterations = iters;
             SP_CUDA_TRY(cudaMemcpyAsync(d_one, &c, sizeof(int), cudaMemcpyHostToDevice, st));
-            SP_CUDA_TRY(cudaMemcpyAsync(b->args.a_v + I.nz, b->av0 + I.nz, sizeof(double) * I.nnz,
-                                        cudaMemcpyDeviceToDevice, st));
-            SP_CUDA_TRY(cudaMemcpyAsync(b->args.t_v + I.nz, b->tv0 + I.nz, sizeof(double) * I.nnz,
-                                        cudaMemcpyDeviceToDevice, st));
             SP_CUDA_TRY(cudaMemsetAsync(b->d_counter, 0, BATCH_COUNTERS * sizeof(int), st));
             SP_CUDA_TRY(cudaEventRecord(e0, st));
             k_batch<NT><<<1, NT, b->smem, st>>>(A2);
@@ -857,8 +853,14 @@ int batch_create(sp_ctx *ctx, const sp_lp *lps, int count, const sp_solver_param
     BatchRes R{};
     ResBatchClass classes[RES_CLASSES] = {};
     if ((rc = upload_resident(b, onchip, all, &R, classes))) return bail(rc, "sp_batch_create: on-chip plans");
-    // one graph: reset the counters, then the on-chip classes (the largest instances first) and,
-    // where instances are left to it, the tuned kernel on values restored as given, side by side
+    // one graph: reset the counters, then side by side the tuned kernel, whose instances are the
+    // largest and take longest, and the on-chip classes, the largest instances first. The on-chip
+    // kernels hold whole SMs until their class has run out, so the tuned kernel is launched, and
+    // has its SMs, before them: 500 LPs of 100-1,900 rows with 40 of 2,200-4,500 take 1,180 ms
+    // (3,000 iterations; alone 99 and 1,110), 1,560 with the tuned kernel behind the others and
+    // the copies of all values that it had to wait for. With 4 of the large ones 827 and 898
+    // (alone 637 and 99): beside kernels that use all of the shared memory the tuned kernel has
+    // less L1 for its local memory.
     cudaGraph_t g;
     SP_CUDA_TRY(cudaStreamSynchronize(st));
     SideStreams side;
@@ -867,17 +869,13 @@ int batch_create(sp_ctx *ctx, const sp_lp *lps, int count, const sp_solver_param
     cudaMemsetAsync(d_counter, 0, BATCH_COUNTERS * sizeof(int), st);
     cudaMemsetAsync(A.drain_ns, 0, sizeof(unsigned long long), st);
     cudaEventRecord(side.fork, st);
+    if (A.count > 0) k_batch<NT><<<b->grid, NT, smem, st>>>(A);
     int launch_rc = SP_OK;
     for (int k = RES_CLASSES - 1; k >= 0; --k) {
         if (classes[k].count == 0) continue;
         cudaStreamWaitEvent(side.st[k], side.fork, 0);
         if (!launch_rc) launch_rc = launch_resident(b, R, classes[k], k, side.st[k]);
         cudaEventRecord(side.done[k], side.st[k]);
-    }
-    if (A.count > 0) {
-        cudaMemcpyAsync(av, av0, sizeof(double) * nz, cudaMemcpyDeviceToDevice, st);
-        cudaMemcpyAsync(tv, tv0, sizeof(double) * nz, cudaMemcpyDeviceToDevice, st);
-        k_batch<NT><<<b->grid, NT, smem, st>>>(A);
     }
     for (int k = 0; k < RES_CLASSES; ++k)
         if (classes[k].count) cudaStreamWaitEvent(st, side.done[k], 0);

@@ -353,7 +353,12 @@ __device__ void batch_solve_one(const BatchArgs &A, int id, double *sh, DevState
     const int tid = threadIdx.x;
     const bool mixed = A.mixed != 0;
 
-    // ---------------- scaling passes (ScaledProblem::new)
+    // ---------------- the values as given (the passes scale them in place), then the scaling
+    // passes (ScaledProblem::new)
+    for (int k = tid; k < I.nnz; k += BT) {
+        av[k] = A.av0[I.nz + k];
+        tv[k] = A.tv0[I.nz + k];
+    }
     for (int i = tid; i < m; i += BT) rs[i] = 1.0;
     for (int j = tid; j < n; j += BT) cs[j] = 1.0;
     __syncthreads();

@@ -68,3 +68,22 @@ def test_an_instance_without_a_first_iteration_has_a_zero_solution(m, ctas, gpu_
             assert not x.any() and not y.any()
             assert all(r.status == 3 for i, r in enumerate(res) if i != at)
         b.close()
+
+
+def test_the_largest_instances_run_beside_the_on_chip_ones(gpu_backend):
+    """Instances beyond the on-chip classes start with them, not after them: together both take
+    well under the sum of their times. And each has the result that it has without the
+    others, on every solve (its values are scaled in place)."""
+    p = sp().SolverParams(tolerance=0.0, infeasibility_tolerance=0.0, max_iterations=1000)
+    small = [sp().generate_random_lp(600 + i, 1000, 2000, (3, 8)) for i in range(1200)]
+    large = [sp().generate_random_lp(2300 + i, 2100 + 10 * i, 4200, (1, 2)) for i in range(4)]
+    took, sols = {}, {}
+    for name, lps in (("small", small), ("large", large), ("both", small + large)):
+        b = sp().BatchSolver(lps, p, gpu_backend)
+        assert [b.engine(i) is None for i in (0, len(lps) - 1)] == [name == "large", name != "small"]
+        took[name] = min(b.solve()[1] for _ in range(4))
+        sols[name] = [b.solution(i) for i in range(len(lps))]
+        b.close()
+    for (x, y), (u, v) in zip(sols["both"], sols["small"] + sols["large"]):
+        assert np.array_equal(x, u) and np.array_equal(y, v)
+    assert took["both"] < 0.85 * (took["small"] + took["large"]), took
