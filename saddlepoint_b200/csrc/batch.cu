@@ -898,10 +898,17 @@ extern "C" int sp_batch_solve(sp_batch *b, sp_batch_result *results, double *ela
     int rc = enter(b->ctx);
     if (rc) return rc;
     cudaStream_t st = b->ctx->stream;
-    {
-        std::lock_guard<std::mutex> lock(b->dl_mu);  // what was fetched of the last solve is stale
-        b->dl_first = b->dl_end = b->dl_next = 0;
-    }
+    // what was fetched of the last solve is stale now, and what another thread fetches during this
+    // one will be (the hand-off's results come after the kernels')
+    struct Stale {
+        sp_batch *b;
+        explicit Stale(sp_batch *batch) : b(batch) { forget(); }
+        ~Stale() { forget(); }
+        void forget() {
+            std::lock_guard<std::mutex> lock(b->dl_mu);
+            b->dl_first = b->dl_end = b->dl_next = 0;
+        }
+    } stale(b);
     EventPair ep;
     if ((rc = ep.init())) return rc;
     SP_CUDA_TRY(cudaEventRecord(ep.e0, st));

@@ -3,6 +3,8 @@
 An instance's class (csrc/batch.cu: res_class) follows from its rows' lengths alone; the result
 of an instance on chip is the solo solve's, bit for bit.
 """
+import threading
+
 import numpy as np
 import pytest
 
@@ -87,3 +89,25 @@ def test_the_largest_instances_run_beside_the_on_chip_ones(gpu_backend):
     for (x, y), (u, v) in zip(sols["both"], sols["small"] + sols["large"]):
         assert np.array_equal(x, u) and np.array_equal(y, v)
     assert took["both"] < 0.85 * (took["small"] + took["large"]), took
+
+
+def test_solutions_read_during_a_solve_do_not_outlive_it(gpu_backend, monkeypatch):
+    """A thread that asks for solutions while another solves gets what is there; afterwards the
+    solutions are the solve's, those of handed-off instances included."""
+    monkeypatch.setenv("SP_BATCH_HANDOFF_S", "1e-9")
+    lps = [sp().generate_random_lp(900 + i, 300 + 200 * i, 600 + 400 * i, (3, 8)) for i in range(4)]
+    p = sp().SolverParams(tolerance=0.0, infeasibility_tolerance=0.0, max_iterations=40_000)
+    b = sp().BatchSolver(lps, p, gpu_backend)
+    res = []
+    t = threading.Thread(target=lambda: res.extend(b.solve()[0]))
+    t.start()
+    while t.is_alive():
+        for i in range(len(lps)):
+            b.solution(i)
+    t.join()
+    assert sum(r.handed_off for r in res) >= len(lps) - 1
+    for i, lp in enumerate(lps):
+        solo = sp().solve(lp, p, gpu_backend)
+        x, y = b.solution(i)
+        assert res[i].iterations == solo.iterations and np.array_equal(x, solo.x) and np.array_equal(y, solo.y), i
+    b.close()
