@@ -1277,6 +1277,8 @@ int grid_order(sp_solver *s, const DevCsr &D, const ResSrc<int> &M, const int *f
 // GRID_MAX_NNZ. Transport, whose gathers are consecutive or of a small vector, so that the
 // stream engine's wide loads count: 500k 11.3 | 10.9, 1.6M 31.3 | 26.6, 3.4M 47.7 | 52.9, 8M
 // 96 | 115 (mixed 3.4M 44.5 | 51.3): hence GRID_MAX_LONG for rows of GRID_LONG_ROW on average.
+// Not for columns of that length: the transport LP transposed 500k 16.7 | 11.4, 1.6M 38.3 | 27.8,
+// 3.4M 79.4 | 54.1, 8M 166 | 115 (mixed 134 | 111).
 //
 // The power iteration (ms, launches | grid): 80k 0.88 | 0.48, 200k 3.67 | 2.20, 500k 3.62 | 2.18,
 // 1M 5.35 | 3.80, 2M 5.06 | 4.48, 3M 10.3 | 10.6 (a grid that waits for its SMs). From 1M on the
