@@ -10,6 +10,7 @@
 
 #include <cmath>
 #include <cstdio>
+#include <cstring>
 #include <string>
 
 #include "../../include/saddlepoint_b200.h"
@@ -67,6 +68,39 @@ __device__ __forceinline__ double div_by_positive(double y, double s) {
     const double q = (z ? s : y) / s;
     return z ? y : q;
 }
+
+// y / s for the dual steps of many rows with one positive s: r = 1/s once, then for each y
+// q0 = y·r and two Newton corrections q ← q + (y - s·q)·r with fused multiply-adds. The first
+// makes q faithful; by Markstein's theorem (P. Markstein, "Computation of elementary functions
+// on the IBM RISC System/6000 processor", 1990) the second then gives y / s correctly rounded,
+// as r is the correctly rounded reciprocal and nothing over- or underflows. Outside ±2^400
+// around 1 for s, ±2^500 for y, the division itself is used; a zero y is its own quotient.
+struct SigmaDivisor {
+    double s, r;
+    bool ok;
+    static __host__ __device__ __forceinline__ int high_word(double v) {
+#ifdef __CUDA_ARCH__
+        return __double2hiint(v);
+#else
+        uint64_t b;
+        memcpy(&b, &v, sizeof b);
+        return (int)(b >> 32);
+#endif
+    }
+    __host__ __device__ __forceinline__ explicit SigmaDivisor(double sigma) : s(sigma), r(1.0 / sigma) {
+        ok = sigma >= 0x1p-400 && sigma <= 0x1p400 && (high_word(sigma) & 0xfffff) != 0xfffff;
+    }
+    __host__ __device__ __forceinline__ double operator()(double y) const {
+        const double a = fabs(y);
+        if (ok && (a == 0.0 || (a >= 0x1p-500 && a <= 0x1p500))) {
+            double q = y * r;
+            q = fma(fma(-s, q, y), r, q);
+            q = fma(fma(-s, q, y), r, q);
+            return a == 0.0 ? y : q;
+        }
+        return y / s;
+    }
+};
 
 // ---- warp and block reductions in a fixed order (deterministic) ----
 
