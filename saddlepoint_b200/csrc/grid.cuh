@@ -25,9 +25,9 @@ namespace sp {
 // ends, and the solve is reported as failed. 1.2 µs for 148 CTAs (B200); counting in two levels
 // took 1.7.
 //
-// Whether all CTAs run is found out by the kernel's first wait, grid_start. The last CTA to start
-// decides for the launch; if another has waited GRID_START_NS for it, that one decides against
-// it, by compare-and-swap on one word, and all CTAs return without effect. That happens where
+// Whether all CTAs run is found out by the kernel's first wait, grid_start: all have come to its
+// gate, or one that has waited GRID_START_NS marks the gate, by compare-and-swap with a count
+// short of all, and all CTAs return without effect. That happens where
 // another stream's long kernel (a batch) holds SMs; the host then runs these iterations by
 // launches, which share the SMs (solver.cu: grid_resume). A cooperative launch would wait for
 // that kernel's end: 640 iterations of a 200k-nonzero LP beside a batch of 0.12 s solved over
@@ -40,10 +40,10 @@ namespace sp {
 constexpr unsigned long long GRID_START_NS = 300000ull, GRID_WAIT_NS = 10000000000ull, GRID_SPIN_NS = 100000ull;
 struct GridBar {
     unsigned count, alive;  // alive: 0 once a wait has given up
-    unsigned gate;          // GRID_GO or GRID_LEFT once the launch's fate is decided
+    unsigned gate;          // CTAs that have started, as `count`; GRID_LEFT: the launch is left
 };
 constexpr unsigned GRID_COUNT0 = ~0u;  // all words at a launch's start (one fill)
-constexpr unsigned GRID_LEFT = 0, GRID_GO = 1;
+constexpr unsigned GRID_LEFT = 1u << 30;
 __host__ __device__ constexpr bool grid_before(unsigned count, unsigned target) { return (int)(count - target) < 0; }
 static_assert(grid_before(GRID_COUNT0, GRID_COUNT0 + 148u) && grid_before(147u, 148u) && !grid_before(148u, 148u) &&
                   !grid_before(3u, GRID_COUNT0) && grid_before(0xfffffff0u, 16u),
@@ -63,34 +63,30 @@ __device__ __forceinline__ unsigned ld_acquire(const unsigned *p) {
     return v;
 }
 
-// Whether all CTAs have started, the same answer in all of them: the last one to come decides for
-// it, or the first whose wait for it exceeds `limit` against it.
-__device__ __forceinline__ bool grid_start(GridState &g, unsigned long long limit) {  // g: a shared variable
+// Whether all CTAs have started, the same answer in all of them: yes once gridDim.x have
+// arrived (and `absent` more, a test's that never come), no once one whose wait exceeds `limit`
+// has marked the gate before that.
+__device__ __forceinline__ bool grid_start(GridState &g, unsigned long long limit, unsigned absent) {  // g: a shared variable
     __syncthreads();
     if (threadIdx.x == 0) {
-        g.passed += gridDim.x;
-        unsigned before, gate = GRID_COUNT0;
-        asm volatile("atom.acq_rel.gpu.global.add.u32 %0, [%1], 1;" : "=r"(before) : "l"(&g.bar->count) : "memory");
-        if (before + 1 == g.passed) {
-            __threadfence();  // all CTAs' writes before the decision
-            gate = atomicCAS(&g.bar->gate, GRID_COUNT0, GRID_GO);
-            if (gate == GRID_COUNT0) gate = GRID_GO;
-        }
+        const unsigned all = GRID_COUNT0 + gridDim.x + absent;
+        asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(&g.bar->gate) : "memory");
+        unsigned gate = ld_acquire(&g.bar->gate);
         const unsigned long long t0 = global_ns();
-        while (gate == GRID_COUNT0 && (gate = ld_acquire(&g.bar->gate)) == GRID_COUNT0) {
+        while (gate != all && !(gate & GRID_LEFT)) {
             const unsigned long long waited = global_ns() - t0;
             if (waited >= limit) {
-                gate = atomicCAS(&g.bar->gate, GRID_COUNT0, GRID_LEFT);
-                if (gate == GRID_COUNT0) {
-                    gate = GRID_LEFT;
+                if (atomicCAS(&g.bar->gate, gate, gate | GRID_LEFT) == gate) {
                     g.leader = 1;
-                }
+                    gate |= GRID_LEFT;
+                    break;
+                }  // else another CTA came or left just now
             } else if (waited > GRID_SPIN_NS) {
                 __nanosleep(1000);
             }
+            gate = ld_acquire(&g.bar->gate);
         }
-        __threadfence();  // ... and after it
-        g.left = gate == GRID_LEFT;
+        g.left = gate != all;
     }
     __syncthreads();
     return !g.left;
@@ -158,6 +154,7 @@ struct GridArgs {
     double *contrib, *ppart;        // the power iteration's
     GridBar *bar;                   // all ones before each launch
     unsigned long long start_ns, wait_ns;  // limits of the first wait and of the others
+    unsigned absent;                       // grid_start's
     int mixed;
 };
 
@@ -227,7 +224,11 @@ struct GridEntries {
     }
 };
 
-constexpr int GRID_B = 4;  // entries of a step
+// Entries of a step. µs an iteration at 2 | 4 | 6 | 8 of them: random LP of 200k nonzeros 9.4 | 8.3 |
+// 8.1 | 8.4, 2M 34.2 | 29.2 | 46.0 | 53.5 (6 and 8 spill where entries are in global memory),
+// 12M 155 | 139 | 226 | 297, 10M power law 129 | 109 | 197 | 247; mixed 9.6 | 8.5 | 8.3 | 8.5,
+// 33.3 | 28.2 | 28.0 | 27.3, 150 | 132 | 129 | 138, 125 | 102 | 102 | 105.
+constexpr int GRID_B = 4;
 
 // One step of a warp: GRID_B entries of each lane's row. A row's last step is filled up with
 // padding; a row without entries takes a step too.
@@ -362,10 +363,9 @@ __global__ void __launch_bounds__(RES_BT, 1) k_grid_mid(const __grid_constant__ 
         const DevState *st = a.g.st;
         sh.due = !st->done && LO == (a.mixed && !st->fp64);
     }
-    __syncthreads();
-    if (!sh.due) return;
     const P L = grid_places<VS, ES, PT, PA>(a, LO);
     grid_open(sh, L, a);
+    if (!sh.due) return;
     const VT *vT, *vA;
     VT *gy, *gx;
     if constexpr (LO) {
@@ -462,7 +462,7 @@ __global__ void __launch_bounds__(RES_BT, 1) k_grid_mid(const __grid_constant__ 
         a.y[k] = yn;
         if constexpr (LO) gy[k] = (float)yn;
     };
-    if (!grid_start(sh.grid, a.start_ns)) {  // so far nothing but this engine's own vectors was written
+    if (!grid_start(sh.grid, a.start_ns, a.absent)) {  // so far nothing but this engine's own vectors was written
         if (threadIdx.x == 0 && sh.grid.leader) {
             a.g.st->error = ERR_GRID_BUSY;
             a.g.st->done = 1;
@@ -561,7 +561,7 @@ __global__ void __launch_bounds__(RES_BT, 1) k_grid_power(const __grid_constant_
     double scale = 1.0 / sqrt(s[0]), lambda = 0.0;
     int iters = 0, error = ERR_NONE;
     bool done = false;
-    if (!grid_start(sh.grid, a.start_ns)) {
+    if (!grid_start(sh.grid, a.start_ns, a.absent)) {
         if (threadIdx.x == 0 && sh.grid.leader) {
             a.g.st->error = ERR_GRID_BUSY;
             a.g.st->pi_done = 1;

@@ -1458,9 +1458,10 @@ int grid_build(sp_solver *s, GridPlan &plan_of) {
     a.bar = (GridBar *)(d + bar);
     a.start_ns = GRID_START_NS;
     a.wait_ns = GRID_WAIT_NS;
-    // test knob of the waits' ends: the first wait, or one between passes, gives up at once
+    // test knob of the waits' ends: the first wait is for a CTA that is not there, or a wait between
+    // passes gives up at once
     if (const char *w = getenv("SP_TEST_GRID_WAIT")) {
-        if (!strcmp(w, "start")) a.start_ns = 0;
+        a.absent = !strcmp(w, "start");
         if (!strcmp(w, "pass")) a.wait_ns = 0;
     }
     a.ppart = s->ppart;
@@ -2231,6 +2232,7 @@ extern "C" int sp_solver_reset(sp_solver *s) {
     SP_CUDA_TRY(cudaMemcpyAsync(s->d_st, s->h_st, sizeof(DevState), cudaMemcpyHostToDevice, st));
     SP_CUDA_TRY(cudaStreamSynchronize(st));
     s->launched = 0;
+    s->settled = false;
     s->time_limited = false;
     s->grid_pause = 0;
     s->grid_backoff = GRID_BACKOFF;
@@ -2417,6 +2419,7 @@ bool res_epochs_on(const sp_solver *s) { return s->res_ctas > 0 && s->timing_eve
 
 // Enqueues the next `n` epochs (fewer at the iteration limit) on the on-chip engine.
 int res_launch_next(sp_solver *s, uint64_t n) {
+    s->settled = false;
     uint64_t its = 0, k = 0;
     for (; k < n; ++k) {
         const uint64_t E = next_epoch(s);
@@ -2433,6 +2436,7 @@ int res_launch_next(sp_solver *s, uint64_t n) {
 // grid engine pauses (a second graph would not do: to make one waits for all streams' kernels).
 int launch_epoch(sp_solver *s, int64_t E) {
     cudaStream_t st = s->ctx->stream;
+    s->settled = false;
     if (res_epochs_on(s)) return res_launch_next(s, 1);
     if (s->timing_every > 0 || s->grid_pause > 0) {
         const int rc = enqueue_epoch(s, E, st, s->timing_every > 0, false);
@@ -2482,7 +2486,10 @@ int settle(sp_solver *s, DevState *h) {
         *h = *s->h_st;
         if (h->error == ERR_GRID_STALL) return fail(SP_ERR_CUDA, GRID_STALL_MESSAGE);
         if (h->error == ERR_PIPELINE_STALL) return fail(SP_ERR_CUDA, PIPELINE_STALL_MESSAGE);
-        if (h->error != ERR_GRID_BUSY) return SP_OK;
+        if (h->error != ERR_GRID_BUSY) {
+            s->settled = true;
+            return SP_OK;
+        }
         const uint64_t queued = s->launched;
         if ((rc = grid_resume(s, *h))) return rc;
         while (s->launched < queued)
@@ -2635,7 +2642,7 @@ extern "C" int sp_solver_download(sp_solver *s, double *x, double *y) {
     if (rc) return rc;
     cudaStream_t st = s->ctx->stream;
     DevState h;
-    if ((rc = settle(s, &h))) return rc;
+    if (!s->settled && (rc = settle(s, &h))) return rc;
     if (!s->out_x) {
         if ((rc = dalloc(&s->out_x, s->n)) || (rc = dalloc(&s->out_y, s->m))) return rc;
     }

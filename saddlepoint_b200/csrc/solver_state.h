@@ -87,6 +87,7 @@ struct sp_solver {
     std::map<int64_t, cudaGraphExec_t> graphs;  // epoch length -> instantiated graph
     std::map<int64_t, int64_t> graph_kernels;  // epoch length -> kernel nodes of its graph
     uint64_t launched = 0;
+    bool settled = false;  // the state of everything launched has been looked at (settle)
     bool time_limited = false;
     double setup_s = 0, solve_s = 0;
     double *out_x = nullptr, *out_y = nullptr;

@@ -2,8 +2,8 @@
 
 A launch of the grid engine whose CTAs cannot all start, since other streams' kernels hold SMs, is
 left without effect and its iterations run by launches; the results keep their bits. The test
-knob SP_TEST_GRID_WAIT (read when a solver is created) makes the first wait ("start") or the
-waits between passes ("pass") give up at once.
+knob SP_TEST_GRID_WAIT (read when a solver is created) makes the first wait be for a CTA that is
+not there ("start"), or the waits between passes give up at once ("pass").
 """
 import threading
 import time
