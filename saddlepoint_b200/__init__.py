@@ -264,21 +264,25 @@ class ScaledProblem:
 
 
 class _Handle:
-    """A native object that belongs to a backend's context. The backend keeps a weak
-    reference to each, so closing the backend frees its objects first and a handle
-    never outlives the context it was made on."""
+    """A native object that belongs to a backend's context. The backend keeps what it takes to
+    free each (and a weak reference), so closing the backend frees its objects first and a
+    handle never outlives the context it was made on. Whoever takes an object out of the
+    backend's table frees it: in a garbage cycle Python clears the weak references and runs
+    the backend's and the objects' __del__ in any order."""
 
     _free = ""
 
     def _attach(self, backend: "CudaBackend", handle):
         self.backend, self.h = backend, handle
+        backend._live[handle.value] = self._free
         backend._children.add(self)
 
     def close(self):
         h = getattr(self, "h", None)
         if h:
             self.h = None
-            getattr(library(), self._free)(h)
+            if self.backend._live.pop(h.value, None):
+                getattr(library(), self._free)(h)
 
     def __del__(self):
         self.close()
@@ -324,11 +328,15 @@ class CudaBackend:
             raise BackendError(rc, f"no usable CUDA device {ordinal}")
         self.lib, self.h = lib, h
         self._children = weakref.WeakSet()
+        self._live = {}  # address of each native object -> the function that frees it
 
     def close(self):
         if getattr(self, "h", None):
             for child in list(self._children):
                 child.close()
+            while self._live:
+                address, free = self._live.popitem()
+                getattr(self.lib, free)(C.c_void_p(address))
             self.lib.sp_ctx_destroy(self.h)
             self.h = None
 
