@@ -5,7 +5,7 @@
 // reference's stable counting sort (problem.rs:88-109, bit for bit), plans the instances
 // that run on chip (batch_resident.cuh) in classes by cluster size, picks the SpMV variant
 // of the others with the tuner below, and captures [reset the work counters, launch a
-// persistent kernel per class and one for the others, side by side] as one CUDA graph.
+// persistent kernel for the others and one per class, side by side] as one CUDA graph.
 // sp_batch_solve replays the graph; the scaling, power iteration and PDHG loop of
 // every instance run inside the kernels.
 #include <algorithm>
@@ -241,6 +241,9 @@ ResClass res_class(int k) {
                                                 {4, RES_SMALL_PT, RES_SMALL_PA}};
     return C[k];
 }
+
+// Rows are dealt by cost alone (res_cut), so uneven lengths can overflow one CTA's share near a
+// class's limits; the next class is tried then, and after the last the tuned kernel has it.
 
 // The plans of the instances that run on chip, by class.
 struct ResBatchPlan {

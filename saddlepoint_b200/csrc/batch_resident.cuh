@@ -5,7 +5,9 @@
 //
 // Against the variants of batch_kernels.cuh (one CTA of 256 threads walking tiles or lane
 // groups through L2, each a chain of round trips): the vectors and, where they fit, the
-// entries are read from shared memory, by 16 warps that own their rows.
+// entries are read from shared memory, by 16 warps that own their rows. Entries in L2 (most
+// instances of some 900 rows and more) are what the warps wait for most: their latency, with four warps
+// a scheduler, not the rate of L2 (11 % of it) or of the shared memory (30 %).
 #pragma once
 
 #include "batch_kernels.cuh"

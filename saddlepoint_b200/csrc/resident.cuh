@@ -15,9 +15,10 @@
 // them, and the column indices of the other matrix are renamed to positions, so every row
 // vector is read and written in place of its thread without a permutation.
 //
-// What bounds an iteration here is shared memory (a gather of 32 entries takes about six of
-// its clocks, bank conflicts included) and the chain of instructions of the longest warp, at
-// 4-9 clocks each. So the first entries of each warp's first rows stay in registers; an entry
+// What bounds an iteration here is latency: the chain of instructions of the longest warp, at
+// 4-9 clocks each, shared memory's (a gather of 32 entries takes about six of its clocks, bank
+// conflicts included, which keeps it 30 % busy), L2's where the entries are there, and with a
+// cluster its barrier and the fence of the release. So the first entries of each warp's first rows stay in registers; an entry
 // in shared memory is its value and the place of its vector entry in 16 bits; slots of padding
 // hold -0.0 and the place of a 1.0, so that their product -0.0 changes no sum and the loops
 // carry no predicates; the vectors' places in shared memory are constants of the kernel; and
