@@ -1416,7 +1416,6 @@ int grid_build(sp_solver *s, GridPlan &plan_of) {
     const size_t gathered32 = s->mixed ? room(4 * (N + M + 2 * GRID_ONES)) : 0;
     const size_t contrib = room(8 * N), bar = room(sizeof(GridBar));
     cudaStream_t st = s->ctx->stream;
-    int rc;
     bool room_for = !dmalloc(&s->res_mem, bytes);
     for (int q = 0; q < 6 && room_for; ++q) {  // A's positions, values and FP32 values, then A'ᵀ's
         const size_t slots = (size_t)(q < 3 ? PA : PT).slots, width = q % 3 == 1 ? 8 : 4;
@@ -1468,10 +1467,12 @@ int grid_build(sp_solver *s, GridPlan &plan_of) {
     a.mixed = s->mixed;
     a.g = ptrs_of(s);
     k_grid_ones<<<GRID_ONES / NT, NT, 0, st>>>(a);
-    if ((rc = grid_order(s, s->A, a.A, (const int *)(d + oa.first), ctas, (int *)(d + oa.perm), (int *)(d + oa.inv))) ||
-        (rc = grid_order(s, s->AT, a.T, (const int *)(d + ot.first), ctas, (int *)(d + ot.perm), (int *)(d + ot.inv)))) {
+    if (grid_order(s, s->A, a.A, (const int *)(d + oa.first), ctas, (int *)(d + oa.perm), (int *)(d + oa.inv)) ||
+        grid_order(s, s->AT, a.T, (const int *)(d + ot.first), ctas, (int *)(d + ot.perm), (int *)(d + ot.inv))) {  // no room for the sort
         cudaStreamSynchronize(st);
-        return rc;
+        release_grid(s, st);
+        s->ctx->last_error.clear();
+        return SP_OK;
     }
     const int ta = (int)PA.tasks.size(), tt = (int)PT.tasks.size(), W = NT / 32, most = s->ctx->sms * 16;
     k_res_fill<int><<<std::min(most, (ta + W - 1) / W), NT, 0, st>>>(a.A, ctas, ta, (int)n, GRID_ONES, (const int *)(d + ot.inv), s->A.ci, s->A.v);

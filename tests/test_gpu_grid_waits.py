@@ -42,6 +42,15 @@ def test_epochs_left_to_launches_keep_their_bits(check_every, iters, mixed, left
     assert a.norm_estimate == b.norm_estimate
 
 
+@pytest.mark.parametrize("mixed", [False, True])
+def test_epochs_left_to_the_large_problem_engines_keep_their_bits(mixed, left_at_start, gpu_backend):
+    """1.2M nonzeros: the launches are the stream engine's and the SELL copy's, on two streams."""
+    lp = sp().generate_random_lp(25, 120_000, 240_000, (5, 5))
+    p = params(64 * 5, precision=sp().Precision.Mixed if mixed else sp().Precision.FP64)
+    a, b = solve_with("grid", lp, p, gpu_backend), solve_with("tiles", lp, p, gpu_backend)
+    assert_identical(a, b)
+
+
 @pytest.mark.parametrize("read", ["sync", "info", "download", "trace", "solve"])
 def test_every_read_finds_the_epochs_that_were_left(read, left_at_start, monkeypatch, gpu_backend):
     """Epochs queued behind the one that was left are run too, whatever asks first, with a warm
