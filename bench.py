@@ -295,6 +295,8 @@ def time_form(sp, torch, lp, backend, precision, steps, warmup, dist, device):
     ms = e0.elapsed_time(e1)
     ms_max = dist.max(ms)
     done = solver.info().iterations
+    if solver.epoch_engine()["left"]:
+        raise RuntimeError("epochs were left to launches outside the timed region: another kernel held SMs")
     if done != (warmup + steps) * ITERS_PER_STEP:
         raise RuntimeError(f"the timed solve stopped early: {done} iterations, status {solver.info().status}")
     # launch times of the two fused passes: events around every 4th P/D launch pair of

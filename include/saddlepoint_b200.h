@@ -214,7 +214,9 @@ int sp_solver_reset(sp_solver *s);
  * instead of from 0. No counterpart in the reference, whose solve always starts at 0. */
 int sp_solver_warm_start(sp_solver *s, const double *x, const double *y);
 /* Enqueues `epochs` epochs of check_every iterations without waiting; a converged
- * state turns further epochs into no-ops. */
+ * state turns further epochs into no-ops. Epochs that the grid engine leaves to launches
+ * (sp_solver_epoch_engine) run when the state is next read: by the functions below, a solve
+ * or sp_solver_trace. These fail with SP_ERR_CUDA after a wait on the device that gave up. */
 int sp_solver_run_epochs(sp_solver *s, uint64_t epochs);
 int sp_solver_sync(sp_solver *s);
 int sp_solver_info(sp_solver *s, sp_solution_info *info);
